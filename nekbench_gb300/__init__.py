@@ -200,6 +200,17 @@ def _require_cuda(*ts):
             raise NekbError(ERR_INVALID, "device arrays must be CUDA tensors")
 
 
+def _require_entries(**needed):
+    """name=(tensor, n): the kernel goes through n entries from the tensor's first on, which its
+    storage has to hold (a raw address is taken as it is)."""
+    for name, (t, n) in needed.items():
+        if isinstance(t, int) or (t.numel() >= n and t.is_contiguous()):
+            continue
+        held = t.untyped_storage().nbytes() // t.element_size() - t.storage_offset()
+        if held < n:
+            raise NekbError(ERR_INVALID, f"{name}: {held} entries from its first on, {n} are needed")
+
+
 # --------------------------------------------------------------------------- axhelm
 def flags_from_name(name: str) -> int:
     f = C.c_int(0)
@@ -563,8 +574,12 @@ def dot_num_blocks(N, block_size=256):
 
 
 def dot_partials(variant, N, w, x, y, wxy, Nfields=1, offset=0, block_size=256, stream=None):
-    """Per-block partials of the dot benchmark kernels (dot/kernel/VOLTA/dot.okl)."""
+    """Per-block partials of the dot benchmark kernels (dot/kernel/VOLTA/dot.okl).  The block
+    variant reads w, x and y alike at node + field * offset (dot.okl:67-111)."""
     _require_cuda(w, x, y, wxy)
+    if N > 0 and not any(t is None for t in (w, x, y, wxy)):
+        n = N + (Nfields - 1) * offset if variant == DOT_BLOCK and Nfields > 1 else N
+        _require_entries(w=(w, n), x=(x, n), y=(y, n), wxy=(wxy, dot_num_blocks(N, block_size)))
     check(lib().nekb_dot_partials(variant, N, Nfields, offset, block_size, _ptr(w), _ptr(x), _ptr(y),
                                   _ptr(wxy), _stream(stream)))
 
