@@ -388,7 +388,7 @@ def prepare(case, seed):
         g = _gen(seed * 7919 + 6)
         n, f = c["n"], c["fields"]
         name = ("weightedInnerProduct2_v0", "weightedInnerProduct2_v1", "weightedBlockInnerProduct2")[c["variant"]]
-        w, x, y = _rand(g, f * n, 0, 1), _rand(g, f * n, -1, 1), _rand(g, f * n, -1, 1)  # w per field too
+        w, x, y = _rand(g, n, 0, 1), _rand(g, f * n, -1, 1), _rand(g, f * n, -1, 1)
         out = torch.zeros(nb.dot_num_blocks(n, c["block"]), dtype=torch.float64, device="cuda")
         s.update(kernel=nb.load_dot_kernel(name, c["block"], f), out=out,
                  args=((n, n) if c["variant"] == 2 else (n,)) + (w, x, y))
@@ -466,7 +466,7 @@ def work(case):
         tensor = n ** 3 * q + n ** 2 * q ** 2 + n * q ** 3
         return {"bytes": 8 * c["E"] * (10 * q ** 3 + 7 * n ** 3),
                 "flops": c["E"] * (12 * tensor + 18 * q ** 4 + 33 * q ** 3 + 3 * n ** 3)}
-    return {"bytes": 8 * (c["n"] * 3 * c["fields"] + c["n"] // c["block"]), "flops": 3 * c["n"] * c["fields"]}
+    return {"bytes": 8 * (c["n"] * (1 + 2 * c["fields"]) + c["n"] // c["block"]), "flops": 3 * c["n"] * c["fields"]}
 
 
 # --------------------------------------------------------------------------- the same in 64 bits, plain torch
@@ -652,8 +652,8 @@ def _exact_adv(c, seed):
 def _exact_dot(c, seed):
     g = _gen(seed * 7919 + 6)
     n, f = c["n"], c["fields"]
-    w, x, y = _rand(g, f * n, 0, 1), _rand(g, f * n, -1, 1), _rand(g, f * n, -1, 1)  # w per field too
-    v = (w * x * y).view(f, n).sum(0)
+    w, x, y = _rand(g, n, 0, 1), _rand(g, f * n, -1, 1), _rand(g, f * n, -1, 1)
+    v = (w * (x * y).view(f, n)).sum(0)
     return torch.nn.functional.pad(v, (0, -n % c["block"])).view(-1, c["block"]).sum(1)
 
 
