@@ -14,9 +14,10 @@
 // D^T contributions of a node are aligned to the largest of their exponents, added
 // as integers and rounded to FP64 once.  Four barriers per element and field.
 //
-// An element group whose values cannot be held in fixed point (Inf, NaN, extreme
-// exponents; see fixedpt.cuh), or any element when D cannot, is evaluated with
-// FP64 sums (direct_field).
+// An element whose values cannot be held in fixed point (Inf, NaN, extreme exponents; see
+// fixedpt.cuh) is evaluated with FP64 sums (direct_field), as is every element when D
+// cannot.  The other elements of its CTA go on, so that an element's bits do not depend
+// on those beside it.
 #pragma once
 
 #include "fixedpt.cuh"
@@ -48,8 +49,8 @@ struct CfgFX {
   static constexpr bool EO = NQ >= 6;
   static constexpr int TAB = fx::Table<NQ, false>::size;  // the larger of the two forms' tables
   // two matrix tables, three node arrays per element, line exponents of three
-  // directions, row exponents of the tables
-  static constexpr int SMEM = (2 * TAB + NEL * 3 * AS) * 8 + (NEL * 3 * NQ2 + 2 * NQ) * 4;
+  // directions, row exponents of the tables, a flag per element
+  static constexpr int SMEM = (2 * TAB + NEL * 3 * AS) * 8 + (NEL * 3 * NQ2 + 2 * NQ + NEL) * 4;
   // registers per thread the launch bounds aim at, by measurement (16.8 M nodes, BK;
   // N=7: 80 registers 414 us, 72: 430, 96: 440; N=12: 96 registers 846 us, 128: 903)
   static constexpr int REGS = G == 3 || NQ <= 7 ? 64 : NQ == 8 ? 80 : 96;
@@ -153,6 +154,7 @@ template <int NQ, int G>
 struct Place {
   using Cf = CfgFX<NQ, G>;
   double* A;           // node arrays A, B, C of the element
+  int* flag;           // whether the element has no fixed-point form
   int* ex;             // exponents of r line (j,k) at k NQ + j, s line (i,k) at NQ^2 + k NQ + i, t line (i,j)
   int i, j, ij, group;  // column of the node passes, number of its lines
   bool active;
@@ -219,9 +221,15 @@ __device__ __forceinline__ void output(const Place<NQ, G>& w, int k, const doubl
   Aqe[k * NQ2] = out;
 }
 
-// one field of one element group; false: it has to be evaluated in FP64
+// elements that have to be evaluated in FP64: any of the CTA's (the same in every thread),
+// the thread's own
+struct Refused {
+  bool any, own;
+};
+
+// one field of the CTA's elements
 template <int NQ, int G, bool BK, bool EO>
-__device__ __forceinline__ bool fixed_field(const AxArgs& a, int f, int64_t element, const Place<NQ, G>& w,
+__device__ __forceinline__ Refused fixed_field(const AxArgs& a, int f, int64_t element, const Place<NQ, G>& w,
                                             const Tables& tab)
 {
   using Cf = CfgFX<NQ, G>;
@@ -233,8 +241,22 @@ __device__ __forceinline__ bool fixed_field(const AxArgs& a, int f, int64_t elem
   const double* qe = static_cast<const double*>(a.q) + f * a.offset + element * NP + w.ij;
   double* Aqe = static_cast<double*>(a.Aq) + f * a.offset + element * NP + w.ij;
   double* node = w.node();
-  bool ok = true;
+  bool ok = true, on = w.active;
+  Refused refused{false, false};
   fx::Line<NQ, EO> t;  // G = 1: the thread's t line
+
+  // barrier, after which the elements with a line that is not ok drop out
+  auto agree = [&]() {
+    if (__syncthreads_or(!ok)) {
+      refused = {true, true};
+      if constexpr (Cf::NEL > 1) {
+        if (!ok) *w.flag = 1;
+        __syncthreads();
+        refused.own = *w.flag != 0;
+      }
+      on = on && !refused.own;
+    }
+  };
 
   // the contractions of the lines in shared memory (all of the element's, G = 3)
   auto lines = [&](const int2* tb) {
@@ -266,7 +288,7 @@ __device__ __forceinline__ bool fixed_field(const AxArgs& a, int f, int64_t elem
     }
   };
 
-  if (w.active) {
+  if (on) {
     if constexpr (G == 1) {
       double r_q[NQ];
 #pragma unroll
@@ -291,16 +313,17 @@ __device__ __forceinline__ bool fixed_field(const AxArgs& a, int f, int64_t elem
     }
   }
   __syncthreads();
-  if (w.active) lines(tab.d);
-  if (__syncthreads_or(!ok)) return false;
-  if (w.active) {
+  if (on) lines(tab.d);
+  agree();
+  if (Cf::NEL == 1 && refused.any) return refused;
+  if (on) {
     const int di = tab.de[w.i], dj = tab.de[w.j];
     nodes(tab.d, [&](int k, long long rt, int te) {
       geometry<NQ, G, BK>(w, k, ge, lam, di, dj, rt, te + tab.de[k]);
     });
   }
   __syncthreads();
-  if (w.active) {
+  if (on) {
     lines(tab.dt);
     if constexpr (G == 1) {
       double gt[NQ];
@@ -309,14 +332,15 @@ __device__ __forceinline__ bool fixed_field(const AxArgs& a, int f, int64_t elem
       ok = t.set(gt) && ok;
     }
   }
-  if (__syncthreads_or(!ok)) return false;
-  if (w.active) {
+  agree();
+  if (Cf::NEL == 1 && refused.any) return refused;
+  if (on) {
     const int di = tab.dte[w.i], dj = tab.dte[w.j];
     nodes(tab.dt, [&](int k, long long rt, int te) {
       output<NQ, G, BK>(w, k, ge, lam + a.offset, qe, Aqe, di, dj, rt, te + tab.dte[k]);
     });
   }
-  return true;
+  return refused;
 }
 
 template <int NQ, int NF, bool BK, bool PARTIAL, int G>
@@ -334,8 +358,10 @@ k_axhelm_fx(const AxArgs a, int64_t groups)
   int* s_exp = reinterpret_cast<int*>(s_all + NEL * 3 * Cf::AS);
   int* s_de = s_exp + NEL * 3 * NQ2;  // row exponents of D and of D^T
   int* s_dte = s_de + NQ;
+  int* s_flag = s_dte + NQ;
 
   const int tid = threadIdx.x;
+  if (tid < NEL) s_flag[tid] = 0;
   const double* D = static_cast<const double*>(a.D);
   bool d_ok, sym;
   const int de = fx::matrix_exponents<NQ>(D, s_de, s_dte, d_ok, sym);
@@ -358,6 +384,7 @@ k_axhelm_fx(const AxArgs a, int64_t groups)
   w.j = w.ij / NQ;
   w.A = s_all + elc * 3 * Cf::AS;
   w.ex = s_exp + elc * 3 * NQ2;
+  w.flag = s_flag + elc;
 
   for (int64_t g = blockIdx.x; g < groups; g += gridDim.x) {
     const int64_t eidx = g * NEL + el;
@@ -367,16 +394,18 @@ k_axhelm_fx(const AxArgs a, int64_t groups)
 #pragma unroll 1
     for (int f = 0; f < NF; ++f) {
       __syncthreads();  // the tables are written; the previous element's or field's last reads
-      bool done = false;
+      Refused refused{true, true};
       if (d_ok) {
         if (Cf::EO && sym)
-          done = fixed_field<NQ, G, BK, Cf::EO>(a, f, element, w, tab);
+          refused = fixed_field<NQ, G, BK, Cf::EO>(a, f, element, w, tab);
         else
-          done = fixed_field<NQ, G, BK, false>(a, f, element, w, tab);
+          refused = fixed_field<NQ, G, BK, false>(a, f, element, w, tab);
       }
-      if (!done)
-        direct_field<NQ, BK>(a, f, element, w.i, w.j, w.active && w.group == 0, w.A, w.A + Cf::AS,
-                             w.A + 2 * Cf::AS);
+      if (refused.any) {
+        direct_field<NQ, BK>(a, f, element, w.i, w.j, w.active && refused.own && w.group == 0, w.A,
+                             w.A + Cf::AS, w.A + 2 * Cf::AS);
+        if (tid < NEL) s_flag[tid] = 0;  // read before direct_field's barriers
+      }
     }
   }
 }
