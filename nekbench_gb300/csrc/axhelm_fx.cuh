@@ -14,10 +14,10 @@
 // D^T contributions of a node are aligned to the largest of their exponents, added
 // as integers and rounded to FP64 once.  Four barriers per element and field.
 //
-// An element whose values cannot be held in fixed point (Inf, NaN, extreme exponents; see
-// fixedpt.cuh) is evaluated with FP64 sums (direct_field), as is every element when D
-// cannot.  The other elements of its CTA go on, so that an element's bits do not depend
-// on those beside it.
+// An element whose values cannot be held in fixed point (Inf, NaN, extreme exponents, in
+// the full-length form a line with one dominating value; see fixedpt.cuh) is evaluated
+// with FP64 sums (direct_field), as is every element when D cannot.  The other elements of
+// its CTA go on, so that an element's bits do not depend on those beside it.
 #pragma once
 
 #include "fixedpt.cuh"
@@ -363,8 +363,9 @@ k_axhelm_fx(const AxArgs a, int64_t groups)
   const int tid = threadIdx.x;
   if (tid < NEL) s_flag[tid] = 0;
   const double* D = static_cast<const double*>(a.D);
-  bool d_ok, sym;
-  const int de = fx::matrix_exponents<NQ>(D, s_de, s_dte, d_ok, sym);
+  bool d_ok, sym, dense;
+  const int de = fx::matrix_exponents<NQ>(D, s_de, s_dte, d_ok, sym, dense);
+  d_ok = d_ok && ((Cf::EO && sym) || dense);
   if (Cf::EO && sym) {
     fx::fill_table<NQ, Cf::EO>(D, de, false, s_D);
     fx::fill_table<NQ, Cf::EO>(D, de, true, s_Dt);

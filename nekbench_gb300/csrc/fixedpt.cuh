@@ -7,8 +7,8 @@
 // bits, seven more than an FP64 mantissa; each row of the matrix likewise.  Both
 // are split into a signed high and a signed low 32-bit word, and
 //   sum_m D_m V_m = 2^64 sum dh vh + 2^32 (sum dh vl + sum dl vh) + sum dl vl
-// is formed in 64-bit accumulators; the last sum is at most 2^-58 NQ of
-// max|D| max|v| and is dropped.
+// is formed in 64-bit accumulators; the last sum is at most 2^-56 NQ (even-odd form from
+// NQ = 11 on: 2^-55 NQ) of max|D| max|v| and is dropped.
 //
 // Even-odd form (EO).  For nodes symmetric about the element centre (GLL,
 // Gauss) D is centro-antisymmetric, D[p'][m'] = -D[p][m] (p' = NQ-1-p).  With
@@ -42,6 +42,19 @@
 // that element in FP64 instead: a line whose largest exponent is outside
 // [kExpLo, kExpHi] (Inf and NaN among them; a line of zeros is fine), and a
 // matrix with a row or column of such a maximum, or of zeros.
+//
+// Precision.  A result is within (N + 2) 2^-54 of max|D| max|v| of its row and line, where
+// FP64 sums are within N 2^-53 of their own terms, sum_m |D_m| |v_m|.  That makes it the
+// less exact one where the terms are far below max|D| max|v|: where a zero of D (its
+// diagonal) meets a value that dominates its line.  The full-length form therefore refuses a line whose second largest
+// value is not zero and more than 2^lone(N) below the largest, and a matrix with an entry
+// beside its diagonal that is more than 2^kDense below its row's or column's largest: every
+// sum then has terms of 2^-(kDense + lone) max|D| max|v| or more.  (GLL nodes, N=2..4, one
+// node's lambda 1e12 times the others: 5.6e-7 of the terms without the rule, 3e-16 with
+// it.)  The even-odd form has no such rule: it adds v_m and v_m' before the products, as
+// the even-odd sums in FP64 that it stands for did, and they lose 2^-53 of the line's
+// largest value there (steep lines, exp(-20 x): 1e-15 to 3.8e-15 of the terms at N=5..13, this
+// form 1.5e-16 to 1.2e-15).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -51,6 +64,18 @@ namespace fx {
 
 constexpr int kExpLo = 400, kExpHi = 1646;    // biased exponents a line's maximum may have
 constexpr int kDExpLo = 823, kDExpHi = 1223;  // and a row or column of the matrix
+constexpr int kDense = 6;
+
+// Binary orders by which one value of a line of N may exceed all others: lines of uniformly
+// random values pass but for about one in 2^14
+__host__ __device__ constexpr int lone(int N) { return N >= 5 ? 4 : (14 + N - 2) / (N - 1); }
+
+// the largest and the second largest of magnitudes (high words) so far
+__device__ __forceinline__ void top_two(unsigned v, unsigned& first, unsigned& second)
+{
+  second = max(second, min(first, v));
+  first = max(first, v);
+}
 
 template <int NQ, bool EO>
 struct Form {
@@ -103,11 +128,17 @@ struct Line {
   __device__ __forceinline__ bool set(const double (&v)[NQ])
   {
     using F = Form<NQ, EO>;
-    unsigned mx = 0;
+    unsigned mx = 0, second = 0;
 #pragma unroll
-    for (int m = 0; m < NQ; ++m) mx = max(mx, hi_abs(v[m]));
+    for (int m = 0; m < NQ; ++m) {
+      if constexpr (EO)
+        mx = max(mx, hi_abs(v[m]));
+      else
+        top_two(hi_abs(v[m]), mx, second);
+    }
     e = (int)(mx >> 20);
     bool ok = e >= kExpLo && e <= kExpHi;
+    if (!EO) ok = ok && (second == 0u || second + ((unsigned)lone(NQ) << 20) >= mx);
     if (e == 0) {  // a line of zeros is fine, a subnormal maximum is not
       unsigned any = mx;
 #pragma unroll
@@ -237,26 +268,28 @@ __device__ __forceinline__ long long shift_down(long long r, int n)
 // Exponents of the rows and columns of a NQ x NQ row-major matrix, NQ <= 16:
 // lane r holds row r's, lane 16 + c column c's; also stored to de and dte (NQ each)
 // by the first warp.  ok: the matrix can be held.  eo: it is centro-antisymmetric to
-// 2^-46 of its largest entry.  Both are the same in every thread of the block, whose
-// warps are whole.
+// 2^-46 of its largest entry.  dense: no entry beside the diagonal is far below its row's or
+// column's largest.  All are the same in every thread of the block, whose warps are whole.
 template <int NQ>
 __device__ __forceinline__ int matrix_exponents(const double* __restrict__ D, int* de, int* dte, bool& ok,
-                                                bool& eo)
+                                                bool& eo, bool& dense)
 {
   const int lane = threadIdx.x & 31;
   const int rc = lane & 15;
-  unsigned mx = 0, asym = 0;
+  unsigned mx = 0, least = 0x7fffffffu, asym = 0;
   if (rc < NQ) {
     const int base = lane < 16 ? rc * NQ : rc, step = lane < 16 ? 1 : NQ;
 #pragma unroll
     for (int m = 0; m < NQ; ++m) {
       const double v = D[base + m * step];
       mx = max(mx, hi_abs(v));
+      if (m != rc) least = min(least, hi_abs(v));
       if (lane < 16) asym = max(asym, hi_abs(v + D[NQ * NQ - 1 - (base + m)]));
     }
   }
   int e = (int)(mx >> 20);
   ok = __all_sync(0xffffffffu, rc >= NQ || (e >= kDExpLo && e <= kDExpHi));
+  dense = __all_sync(0xffffffffu, rc >= NQ || least + ((unsigned)kDense << 20) >= mx);
   const unsigned big = __reduce_max_sync(0xffffffffu, mx), off = __reduce_max_sync(0xffffffffu, asym);
   eo = off + (46u << 20) <= big;
   // mirror rows are equal up to rounding: one exponent for both
