@@ -15,7 +15,7 @@
 // as integers and rounded to FP64 once.  Four barriers per element and field.
 //
 // An element whose values cannot be held in fixed point (Inf, NaN, extreme exponents, in
-// the full-length form a line with one dominating value; see fixedpt.cuh) is evaluated
+// the full-length form a line with too far a dominating value; see fixedpt.cuh) is evaluated
 // with FP64 sums (direct_field), as is every element when D cannot.  The other elements of
 // its CTA go on, so that an element's bits do not depend on those beside it.
 #pragma once
@@ -68,9 +68,11 @@ __device__ __noinline__ void direct_field(const AxArgs& a, int f, int64_t elemen
   const double* ge = static_cast<const double*>(a.ggeo) + element * 7 * NP + ij;
   const double* lam = static_cast<const double*>(a.lambda);
   const double* qe = static_cast<const double*>(a.q) + f * a.offset + element * NP + ij;
+  constexpr int U = NQ <= 5 ? NQ : 1;  // few elements of a mesh come here: a short chain at the low orders
   double r_q[NQ], r_Gt[NQ];
   __syncthreads();  // the arrays were in use
   if (active) {
+#pragma unroll U
     for (int k = 0; k < NQ; ++k) {
       r_q[k] = qe[k * NQ2];
       A[k * NQ2 + ij] = r_q[k];
@@ -78,9 +80,11 @@ __device__ __noinline__ void direct_field(const AxArgs& a, int f, int64_t elemen
   }
   __syncthreads();
   if (active) {
+#pragma unroll U
     for (int k = 0; k < NQ; ++k) {
       const int n = k * NQ2 + ij;
       double qr = 0, qs = 0, qt = 0;
+#pragma unroll U
       for (int m = 0; m < NQ; ++m) {
         qr += D[i * NQ + m] * A[k * NQ2 + j * NQ + m];
         qs += D[j * NQ + m] * A[k * NQ2 + m * NQ + i];
@@ -106,8 +110,10 @@ __device__ __noinline__ void direct_field(const AxArgs& a, int f, int64_t elemen
   __syncthreads();
   if (active) {
     double* Aqe = static_cast<double*>(a.Aq) + f * a.offset + element * NP + ij;
+#pragma unroll U
     for (int k = 0; k < NQ; ++k) {
       double ar = 0, as = 0, at = 0;
+#pragma unroll U
       for (int m = 0; m < NQ; ++m) {
         ar += D[m * NQ + i] * B[k * NQ2 + j * NQ + m];
         as += D[m * NQ + j] * C[k * NQ2 + m * NQ + i];
@@ -130,7 +136,8 @@ __device__ __forceinline__ bool contract_line(double* line, int stride, const in
   double raw[NQ];
 #pragma unroll
   for (int m = 0; m < NQ; ++m) raw[m] = line[m * stride];
-  const bool ok = v.set(raw);
+  bool ok = v.set(raw);
+  if constexpr (!EO) ok = ok && !fx::out_of_reach<NQ>(tab, NQ, fx::Table<NQ, EO>::stride, v, fx::lone(NQ));
   e = v.e + F::kScale;
   long long* out = reinterpret_cast<long long*>(line);
 #pragma unroll 2
@@ -258,6 +265,11 @@ __device__ __forceinline__ Refused fixed_field(const AxArgs& a, int f, int64_t e
     }
   };
 
+  auto set_t = [&](const double (&v)[NQ], const int2* tb) {
+    bool fine = t.set(v);
+    if constexpr (!EO) fine = fine && !fx::out_of_reach<NQ>(tb, NQ, fx::Table<NQ, EO>::stride, t, fx::lone(NQ));
+    return fine;
+  };
   // the contractions of the lines in shared memory (all of the element's, G = 3)
   auto lines = [&](const int2* tb) {
     if constexpr (G == 1) {
@@ -298,7 +310,7 @@ __device__ __forceinline__ Refused fixed_field(const AxArgs& a, int f, int64_t e
         node[k * PS] = r_q[k];
         node[k * PS + AS] = r_q[k];
       }
-      ok = t.set(r_q);
+      ok = set_t(r_q, tab.d);
     } else {
 #pragma unroll
       for (int k0 = 0; k0 < NQ; k0 += G) {
@@ -329,7 +341,7 @@ __device__ __forceinline__ Refused fixed_field(const AxArgs& a, int f, int64_t e
       double gt[NQ];
 #pragma unroll
       for (int k = 0; k < NQ; ++k) gt[k] = node[k * PS + 2 * AS];
-      ok = t.set(gt) && ok;
+      ok = set_t(gt, tab.dt) && ok;
     }
   }
   agree();

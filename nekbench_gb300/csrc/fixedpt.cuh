@@ -46,11 +46,12 @@
 // Precision.  A result is within (N + 2) 2^-54 of max|D| max|v| of its row and line, where
 // FP64 sums are within N 2^-53 of their own terms, sum_m |D_m| |v_m|.  That makes it the
 // less exact one where the terms are far below max|D| max|v|: where a zero of D (its
-// diagonal) meets a value that dominates its line.  The full-length form therefore refuses a line whose second largest
-// value is not zero and more than 2^lone(N) below the largest, and a matrix with an entry
-// beside its diagonal that is more than 2^kDense below its row's or column's largest: every
-// sum then has terms of 2^-(kDense + lone) max|D| max|v| or more.  (GLL nodes, N=2..4, one
-// node's lambda 1e12 times the others: 5.6e-7 of the terms without the rule, 3e-16 with
+// diagonal) meets a value that dominates its line.  The full-length form therefore refuses
+// a line with a row whose terms are below 2^-kReach max|D| max|v| (out_of_reach, looked at only
+// where one value is 2^lone(N) above all others), and a matrix with an entry beside its
+// diagonal (N = 2: any entry, and no line is looked at) that is more than 2^kDense below its
+// row's or column's largest.  (GLL nodes, N=2..4,
+// one node's lambda 1e12 times the others: 5.6e-7 of the terms without the rule, 3e-16 with
 // it.)  The even-odd form has no such rule: it adds v_m and v_m' before the products, as
 // the even-odd sums in FP64 that it stands for did, and they lose 2^-53 of the line's
 // largest value there (steep lines, exp(-20 x): 1e-15 to 3.8e-15 of the terms at N=5..13, this
@@ -64,10 +65,10 @@ namespace fx {
 
 constexpr int kExpLo = 400, kExpHi = 1646;    // biased exponents a line's maximum may have
 constexpr int kDExpLo = 823, kDExpHi = 1223;  // and a row or column of the matrix
-constexpr int kDense = 6;
+constexpr int kDense = 6, kReach = 9;
 
-// Binary orders by which one value of a line of N may exceed all others: lines of uniformly
-// random values pass but for about one in 2^14
+// Binary orders by which one value of a line of N may exceed all others before its rows are
+// looked at (one in 2^14 lines of uniformly random values)
 __host__ __device__ constexpr int lone(int N) { return N >= 5 ? 4 : (14 + N - 2) / (N - 1); }
 
 // the largest and the second largest of magnitudes (high words) so far
@@ -122,7 +123,8 @@ __device__ __forceinline__ void words(long long v, int& hi, int& lo)
 template <int NQ, bool EO>
 struct Line {
   int h[NQ], l[NQ];
-  int e;  // biased exponent of the block
+  int e;         // biased exponent of the block
+  unsigned gap;  // the largest value's high word less the second largest's, 0 if that is a zero (full-length form)
 
   // returns whether the line can be held in fixed point
   __device__ __forceinline__ bool set(const double (&v)[NQ])
@@ -131,14 +133,14 @@ struct Line {
     unsigned mx = 0, second = 0;
 #pragma unroll
     for (int m = 0; m < NQ; ++m) {
-      if constexpr (EO)
+      if constexpr (EO || NQ == 2)
         mx = max(mx, hi_abs(v[m]));
       else
         top_two(hi_abs(v[m]), mx, second);
     }
     e = (int)(mx >> 20);
     bool ok = e >= kExpLo && e <= kExpHi;
-    if (!EO) ok = ok && (second == 0u || second + ((unsigned)lone(NQ) << 20) >= mx);
+    gap = second != 0u ? mx - second : 0u;
     if (e == 0) {  // a line of zeros is fine, a subnormal maximum is not
       unsigned any = mx;
 #pragma unroll
@@ -208,6 +210,30 @@ __device__ __forceinline__ long long dot_part(const int2* row, const Line<NQ, EO
   long long r = (hh << F::kGuard) + (mid >> (32 - F::kGuard));
   if (!F::kOneMid) r += mid2 >> (32 - F::kGuard);
   return r;
+}
+
+// whether some row of a table has too small terms for a line to be held (see above), looked at
+// where one value is more than 2^orders above all others
+template <int N>
+__device__ __forceinline__ bool out_of_reach(const int2* tab, int rows, int stride, const Line<N, false>& v, int orders)
+{
+  if (v.gap <= (unsigned)orders << 20) return false;
+  float top = 0.f;
+#pragma unroll
+  for (int m = 0; m < N; ++m) top = fmaxf(top, fabsf((float)v.h[m]));
+  bool out = false;
+#pragma unroll 1
+  for (int p = 0; p < rows; ++p) {
+    float sum = 0.f, big = 0.f;
+#pragma unroll
+    for (int m = 0; m < N; ++m) {
+      const float d = fabsf((float)tab[p * stride + m].x);
+      big = fmaxf(big, d);
+      sum = fmaf(d, fabsf((float)v.h[m]), sum);
+    }
+    out = out || sum < big * top * (1.f / (1 << kReach));
+  }
+  return out;
 }
 
 // EO: the results of rows p and NQ-1-p (equal for the middle row); else row p
@@ -283,7 +309,7 @@ __device__ __forceinline__ int matrix_exponents(const double* __restrict__ D, in
     for (int m = 0; m < NQ; ++m) {
       const double v = D[base + m * step];
       mx = max(mx, hi_abs(v));
-      if (m != rc) least = min(least, hi_abs(v));
+      if (NQ == 2 || m != rc) least = min(least, hi_abs(v));
       if (lane < 16) asym = max(asym, hi_abs(v + D[NQ * NQ - 1 - (base + m)]));
     }
   }

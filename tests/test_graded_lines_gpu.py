@@ -2,11 +2,10 @@
 extended precision (np.longdouble) on the same operands, component by component.
 
 A contraction's result is off by at most (Nq + 2) 2^-54 of max|D| max|v| of its row and line.
-Where the full-length form is taken (Nq <= 5, or a D without centro-antisymmetry) a line whose
-second largest value is far below the largest goes to the FP64 sums, and what is left has
-terms of 2^-lone 2^-r max|D| max|v| or more, r the binary orders between a row's entries; for
-GLL nodes lone + r <= 7.3 at N = 2, 3, 4.  So each of the operator's two contractions is off by at
-most 7 * 2^-54 * 2^7.3 = 6.2e-14 of its terms, the rest by a few 2^-53: 1.3e-13."""
+Where the full-length form is taken (Nq <= 5, or a D without centro-antisymmetry) that is
+Nq (2^-56 + 2^-58) + 2^-57, 9.4e-17 at Nq = 5, and a line with a row whose terms are below 2^-9
+max|D| max|v| goes to the FP64 sums.  So each of the operator's two contractions is off by at
+most 9.4e-17 * 2^9 = 4.8e-14 of its terms, the rest by a few 2^-53: below 1.3e-13."""
 import numpy as np
 import pytest
 import torch
@@ -92,7 +91,8 @@ def test_any_matrix_component_by_component(nb, O, dev, N, kind):
         D = D * np.linspace(1.0, 1.5, n)[:, None]
     ref, terms = operator(*(a.astype(LD) for a in (D, g, lam[0], lam[1], q)))
     got = run(nb, dev, N, E, D, g, lam, q)
-    # rows of D up to 2^6 apart in their entries: 12 * 2^-54 * 2^(6 + 4) = 6.8e-13, twice
+    # lines that are not looked at: rows of D up to 2^6 apart in their entries, values 2^4:
+    # 12 * 2^-54 * 2^(6 + 4) = 6.8e-13, twice
     assert np.all(abs(got - ref) <= (1e-14 if kind == "banded" else 1.4e-12) * terms)
 
 
