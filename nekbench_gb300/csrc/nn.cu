@@ -212,8 +212,10 @@ k_net_infer(int64_t Etot, int64_t Efield, const __nv_bfloat16* __restrict__ Wbf,
 // owns one row and four output channels (4 NQ sums): per input channel and (dj, dk)
 // it reads NQ + 2 activations and 12 weights for 12 NQ FMAs.  Weight gradients of the
 // middle layer: a thread owns four output channels, one input channel and one dk with
-// all nine (di, dj) taps (36 sums, in registers over all elements of the CTA) and
-// slides along j, so that a row read serves three taps.  Pre-activation derivatives
+// all nine (di, dj) taps (36 sums in registers) and slides along j, so that a row read
+// serves three taps.  An element's sums are formed on their own and then added to the CTA's,
+// which stay in L2 (31 KB at C = 16): a chain of FP32 additions over all nodes of all elements
+// of the CTA would lose digits as the batch grows.  Pre-activation derivatives
 // stay in the registers of the thread that owns them; the loss gradient replaces the
 // activations it no longer needs.  At Nq = 8, C = 16 (256 threads, one CTA per SM) the FMA
 // pipe and the shared-memory return path are about equally loaded.
@@ -432,9 +434,10 @@ k_net_train(int64_t E, const float* __restrict__ W, const float* __restrict__ in
   const bool act = row < T::NQ2;
   const int j = act ? row % NQ : 0, k = act ? row / NQ : 0;
   const int at = (act ? row : 0) * RS;  // the thread's row in an array
-  float w2sum[T::IT2][4][9] = {}, w1sum[T::IT1][3] = {}, w3sum[T::IT1][3] = {};
+  float* gp = gpart + (int64_t)blockIdx.x * P;  // the CTA's sums, in gradient_entry's order
   float lsum = 0.f;
   for (int64_t e = blockIdx.x; e < E; e += gridDim.x) {
+    auto fold = [&](int at, float v) { gp[at] = e < gridDim.x ? v : gp[at] + v; };
     for (int n = tid; n < NP; n += T::THREADS) A0[(n / NQ) * RS + n % NQ] = in[e * NP + n];
     __syncthreads();
     float acc[4][NQ], d1[4][NQ], d2[4][NQ];
@@ -491,19 +494,26 @@ k_net_train(int64_t E, const float* __restrict__ W, const float* __restrict__ in
         for (int o = G / 2; o > 0; o >>= 1) y[i] += __shfl_xor_sync(0xffffffffu, y[i], o);
       }
       if (act && cg == 0) {
+        float lrow = 0.f;
 #pragma unroll
         for (int i = 0; i < NQ; ++i) {
           const float d = y[i] - target[e * NP + row * NQ + i];
-          lsum += d * d;
+          lrow += d * d;
           Gy[at + i] = gscale * d;  // d loss / d y
         }
+        lsum += lrow;
       }
     }
     __syncthreads();
 #pragma unroll
     for (int u = 0; u < T::IT1; ++u) {
       const int n = tid + u * T::THREADS;
-      if (n < C * 9) wgrad_rows<NQ, C>(Gy, A2 + (n / 9) * CS, n % 9, w3sum[u]);
+      if (n < C * 9) {
+        float sum[3] = {};
+        wgrad_rows<NQ, C>(Gy, A2 + (n / 9) * CS, n % 9, sum);
+#pragma unroll
+        for (int di = 0; di < 3; ++di) fold(o3 + di * (C * 9) + n, sum[di]);
+      }
     }
     conv_row4<NQ, C, 1, C>(Gy, zero, sW3b, j, k, cg, acc);
     __syncthreads();  // the activations of layer 2 are read: its gradient takes their place
@@ -519,8 +529,14 @@ k_net_train(int64_t E, const float* __restrict__ W, const float* __restrict__ in
 #pragma unroll
     for (int u = 0; u < T::IT2; ++u) {
       const int n = tid + u * T::THREADS;  // (dk, ci, group of output channels)
-      if (n < G * C * 3)
-        wgrad_plane4<NQ, C>(A2 + (n % G) * CS, A1 + (n / G % C) * CS, zero, n / (G * C) - 1, w2sum[u]);
+      if (n < G * C * 3) {
+        float sum[4][9] = {};
+        wgrad_plane4<NQ, C>(A2 + (n % G) * CS, A1 + (n / G % C) * CS, zero, n / (G * C) - 1, sum);
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+#pragma unroll
+          for (int t = 0; t < 9; ++t) fold(o2 + (9 * q + t) * (G * C * 3) + n, sum[q][t]);
+      }
     }
     conv_row4<NQ, C, C, C>(A2, zero, sW2b, j, k, cg, acc);
     __syncthreads();
@@ -536,40 +552,35 @@ k_net_train(int64_t E, const float* __restrict__ W, const float* __restrict__ in
 #pragma unroll
     for (int u = 0; u < T::IT1; ++u) {
       const int n = tid + u * T::THREADS;
-      if (n < C * 9) wgrad_rows<NQ, C>(A1 + (n / 9) * CS, A0, n % 9, w1sum[u]);
-    }
-    __syncthreads();
-  }
-  float* gp = gpart + (int64_t)blockIdx.x * P;
+      if (n < C * 9) {
+        float sum[3] = {};
+        wgrad_rows<NQ, C>(A1 + (n / 9) * CS, A0, n % 9, sum);
 #pragma unroll
-  for (int u = 0; u < T::IT1; ++u) {
-    const int n = tid + u * T::THREADS;
-    if (n < C * 9) {
-#pragma unroll
-      for (int di = 0; di < 3; ++di) {
-        gp[(n / 9) * kTaps + 3 * (n % 9) + di] = w1sum[u][di];
-        gp[o3 + (n / 9) * kTaps + 3 * (n % 9) + di] = w3sum[u][di];
+        for (int di = 0; di < 3; ++di) fold(di * (C * 9) + n, sum[di]);
       }
     }
-  }
-#pragma unroll
-  for (int u = 0; u < T::IT2; ++u) {
-    const int n = tid + u * T::THREADS;
-    if (n < G * C * 3) {
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-#pragma unroll
-        for (int t = 0; t < 9; ++t)
-          gp[o2 + ((n % G + q * G) * C + n / G % C) * kTaps + 9 * (n / (G * C)) + t] = w2sum[u][q][t];
-    }
+    __syncthreads();
   }
   const float ls = block_sum_f(lsum, red);
   if (tid == 0) lpart[blockIdx.x] = ls;
 }
 
-// grad[p] = sum_b gpart[b][p], loss likewise: 32 parameters per CTA, eight runs of blocks
-// each, summed in order and then over the runs
-__global__ void __launch_bounds__(256) k_net_reduce(int P, int nb, const float* __restrict__ gpart,
+// the weight that entry p of a CTA's sums belongs to: there neighbouring threads of
+// k_net_train hold neighbouring entries
+__device__ __forceinline__ int gradient_entry(int p, int C)
+{
+  const int o2 = kTaps * C, o3 = o2 + kTaps * C * C, G = C / 4;
+  if (p >= o2 && p < o3) {
+    const int m = p - o2, n = m % (G * C * 3), v = m / (G * C * 3), q = v / 9, t = v % 9;
+    return o2 + ((n % G + q * G) * C + n / G % C) * kTaps + 9 * (n / (G * C)) + t;
+  }
+  const int base = p < o2 ? 0 : o3, n = (p - base) % (C * 9), di = (p - base) / (C * 9);
+  return base + (n / 9) * kTaps + 3 * (n % 9) + di;
+}
+
+// grad = sum over blocks of their sums, loss likewise: 32 parameters per CTA, eight runs of
+// blocks each, summed in order and then over the runs
+__global__ void __launch_bounds__(256) k_net_reduce(int P, int C, int nb, const float* __restrict__ gpart,
                                                     const float* __restrict__ lpart, float* __restrict__ grad,
                                                     float* __restrict__ loss, float lscale)
 {
@@ -585,7 +596,7 @@ __global__ void __launch_bounds__(256) k_net_reduce(int P, int nb, const float* 
   __syncthreads();
   if (run == 0) {
     for (int r = 1; r < 8; ++r) s += sh[r][lane];
-    if (p < P) grad[p] = s;
+    if (p < P) grad[gradient_entry(p, C)] = s;
   }
   if (blockIdx.x == 0 && run == 1) {
     float v = 0.f;
@@ -809,7 +820,7 @@ int run_train(nekb_net* net, int64_t E, const float* in, const float* target, cu
   k_net_train<NQ, C><<<(unsigned)grid, TrainCfg<NQ, C>::THREADS, SM, s>>>(
       E, net->W.as<float>(), in, target, gscale, net->gpart.as<float>(), net->lpart.as<float>());
   NEKB_CUDA(cudaGetLastError());
-  k_net_reduce<<<(net->P + 31) / 32, 256, 0, s>>>(net->P, (int)grid, net->gpart.as<float>(),
+  k_net_reduce<<<(net->P + 31) / 32, 256, 0, s>>>(net->P, C, (int)grid, net->gpart.as<float>(),
                                                   net->lpart.as<float>(), net->grad.as<float>(),
                                                   net->loss.as<float>(), 1.0f / (float)(E * np_of(NQ)));
   NEKB_CUDA(cudaGetLastError());
