@@ -24,7 +24,14 @@
 // changed nothing.
 //
 // An element with values that have no fixed-point form, and all elements when a matrix
-// has none, are evaluated with FP64 sums (direct).
+// has none, are evaluated with FP64 sums (direct).  A line shares one exponent, so where a
+// zero of a matrix meets a value far above the others the result would be short of bits
+// (fixedpt.cuh).  The node that odd Gauss and Gauss-Lobatto grids share, the centre, has such
+// zeros in the interpolation beside it and in the derivative on the diagonal: an element with
+// a line to be derived or projected that has too small terms there takes the FP64 sums too.
+// So do all elements when zeros stand in more than one row, as when the cubature nodes are the
+// element's own (the interpolation is then the identity, and every value small beside its
+// line's largest would lose).
 #pragma once
 #include "adv_impl.cuh"
 #include "fixedpt.cuh"
@@ -37,6 +44,12 @@ using namespace adv;
 // exponents (biased) of the largest entry of a line of U and of a matrix row: three
 // interpolations, the metric terms and three projections stay in the normal range
 constexpr int kULo = 500, kUHi = 1546, kMLo = 983, kMHi = 1063;
+// binary orders below its row's largest from which an entry counts as a zero (Gauss-Lobatto
+// to Gauss interpolation has entries 10 orders below)
+constexpr int kZero = 12;
+// binary orders by which one value of a line of N may exceed all others before its rows are
+// looked at
+__host__ __device__ constexpr int far(int N) { return N >= 8 ? 6 : N >= 6 ? 7 : N >= 4 ? 8 : 10; }
 
 template <int NQ, int CQ>
 struct Shape {
@@ -74,19 +87,26 @@ struct Ln : fx::Line<N, false> {
   __device__ __forceinline__ void from(const long long (&r)[N], const int (&e)[N])
   {
     long long m[N];
-    int ex[N], top = -100000;
+    int ex[N], top = -100000, second = -100000;
 #pragma unroll
     for (int a = 0; a < N; ++a) {
       const int lz = __clzll(r[a] ^ (r[a] >> 63));  // 1..64
       ex[a] = lz == 64 ? -100000 : e[a] - (lz - 1);
       m[a] = lz == 64 ? 0 : r[a];
       asm("shl.b64 %0, %0, %1;" : "+l"(m[a]) : "r"(lz - 1));
+      if (N > 2) second = max(second, min(top, ex[a]));
       top = max(top, ex[a]);
     }
     constexpr int down = 10 - F::kVUp;  // 63-bit magnitudes to 53 + kVUp bits
 #pragma unroll
     for (int a = 0; a < N; ++a) fx::words(fx::shift_nearest(m[a], min(top - ex[a], 1000) + down), this->h[a], this->l[a]);
     x = max(top, -50000) + down;
+    this->gap = second == -100000 ? 0u : (unsigned)(top - second) << 20;
+  }
+  // whether every row of a table has terms for which the line can be held
+  __device__ __forceinline__ bool fits(const int2* tab, int rows, int stride) const
+  {
+    return !fx::out_of_reach<N>(tab, rows, stride, *this, far(N));
   }
   // row of a table times the line; result exponent: x + row exponent + kOut
   __device__ __forceinline__ long long dot(const int2* row) const
@@ -97,20 +117,29 @@ struct Ln : fx::Line<N, false> {
 };
 
 // Rows (stride RS) of a matrix of ROWS x COLS entries at M[p ps + m ms], with the exponents
-// of their entries (value = entry 2^ex) in ex; whether every row has a fixed-point form, in
-// every thread.  The block synchronises here.
-template <int ROWS, int COLS, int RS>
+// of their entries (value = entry 2^ex) in ex; whether the matrix has a fixed-point form, in
+// every thread: every row in range, and, with COUNT, zeros (kZero; DIAG: beside the diagonal)
+// in one row at most (two columns: none).  The block synchronises here.
+template <int ROWS, int COLS, int RS, bool COUNT, bool DIAG = false>
 __device__ __forceinline__ bool fill(const double* __restrict__ M, int ps, int ms, int2* t, int* ex)
 {
-  bool ok = true;
-  for (int p = threadIdx.x; p < ROWS; p += blockDim.x) {
-    unsigned mx = 0;
-    for (int m = 0; m < COLS; ++m) mx = max(mx, fx::hi_abs(M[p * ps + m * ms]));
+  static_assert(ROWS <= 32, "one row per thread");
+  bool ok = true, zeros = false;
+  if (threadIdx.x < ROWS) {
+    const int p = threadIdx.x;
+    unsigned mx = 0, least = 0x7fffffffu;
+    for (int m = 0; m < COLS; ++m) {
+      const unsigned v = fx::hi_abs(M[p * ps + m * ms]);
+      mx = max(mx, v);
+      if (!DIAG || COLS == 2 || m != p) least = min(least, v);
+    }
     const int e = (int)(mx >> 20);
     ok = e >= kMLo && e <= kMHi;
+    zeros = least + ((unsigned)kZero << 20) < mx;
     ex[p] = e;
   }
-  const bool all = !__syncthreads_or(!ok);
+  bool all = !__syncthreads_or(!ok);
+  if (COUNT) all = __syncthreads_count(zeros) <= (COLS == 2 ? 0 : 1) && all;
   for (int n = threadIdx.x; n < ROWS * RS; n += blockDim.x) {
     const int p = n / RS, m = n - p * RS;
     int2 w = make_int2(0, 0);
@@ -118,7 +147,7 @@ __device__ __forceinline__ bool fill(const double* __restrict__ M, int ps, int m
     t[n] = w;
   }
   __syncthreads();
-  for (int p = threadIdx.x; p < ROWS; p += blockDim.x) ex[p] -= 1075 + 7;
+  if (threadIdx.x < ROWS) ex[threadIdx.x] -= 1075 + 7;
   return all;
 }
 
@@ -225,9 +254,9 @@ k_adv_fx(int64_t E, const double* __restrict__ vgeo, const double* __restrict__ 
   long long* Hi = reinterpret_cast<long long*>(H);
 
   const int tid = threadIdx.x;
-  bool m_ok = fill<CQ, NQ, S::RN>(cubInterpT, 1, CQ, tI, xI);
-  m_ok = fill<NQ, CQ, S::RQ>(cubInterpT, CQ, 1, tIt, xIt) && m_ok;
-  m_ok = fill<CQ, CQ, S::RQ>(cubD, CQ, 1, tD, xD) && m_ok;
+  bool m_ok = fill<CQ, NQ, S::RN, true>(cubInterpT, 1, CQ, tI, xI);
+  m_ok = fill<NQ, CQ, S::RQ, false>(cubInterpT, CQ, 1, tIt, xIt) && m_ok;
+  m_ok = fill<CQ, CQ, S::RQ, true, true>(cubD, CQ, 1, tD, xD) && m_ok;
 
   // the thread's component and column (i, j); also the numbers of its lines
   const bool act = tid < 3 * CQ2;
@@ -306,6 +335,7 @@ k_adv_fx(int64_t E, const double* __restrict__ vgeo, const double* __restrict__ 
         x[k] = e3[tid] + xI[k];
       }
       t.from(r, x);
+      ok = t.fits(tD, CQ, S::RQ) && ok;
 #pragma unroll 1
       for (int k = f; k < CQ; k += 3) {
         const int n = k * PS + j * LQ + i;
@@ -332,6 +362,7 @@ k_adv_fx(int64_t E, const double* __restrict__ vgeo, const double* __restrict__ 
       }
       Ln<CQ> l;
       l.from(r, x);
+      ok = l.fits(tD, CQ, S::RQ) && ok;
       e1[tid] = l.x + l.kOut;
 #pragma unroll 2
       for (int p = 0; p < CQ; ++p) line[p] = l.dot(tD + p * S::RQ);
@@ -342,6 +373,7 @@ k_adv_fx(int64_t E, const double* __restrict__ vgeo, const double* __restrict__ 
         x[n] = e3[f * CQ2 + n * CQ + i] + xI[j];
       }
       l.from(r, x);
+      ok = l.fits(tD, CQ, S::RQ) && ok;
       e2[tid] = l.x + l.kOut;
 #pragma unroll 2
       for (int p = 0; p < CQ; ++p) line[p * LQ] = l.dot(tD + p * S::RQ);
@@ -362,7 +394,7 @@ k_adv_fx(int64_t E, const double* __restrict__ vgeo, const double* __restrict__ 
 #pragma unroll
       for (int k = 0; k < CQ; ++k) v[k] = A[col + k * PS];
       Ln<CQ> l;
-      ok = l.from(v, fx::kExpLo, fx::kExpHi) && ok;
+      ok = l.from(v, fx::kExpLo, fx::kExpHi) && l.fits(tIt, NQ, S::RQ) && ok;
       e3[tid] = l.x + l.kOut;
 #pragma unroll 2
       for (int c = 0; c < NQ; ++c) Ai[col + c * PS] = l.dot(tIt + c * S::RQ);
@@ -384,6 +416,7 @@ k_adv_fx(int64_t E, const double* __restrict__ vgeo, const double* __restrict__ 
       }
       Ln<CQ> l;
       l.from(r, x);
+      ok = l.fits(tIt, NQ, S::RQ) && ok;
       e1[tid] = l.x + l.kOut;
 #pragma unroll 2
       for (int b = 0; b < NQ; ++b) line[b * LQ] = l.dot(tIt + b * S::RQ);
@@ -402,11 +435,15 @@ k_adv_fx(int64_t E, const double* __restrict__ vgeo, const double* __restrict__ 
       }
       Ln<CQ> l;
       l.from(r, x);
+      ok = l.fits(tIt, NQ, S::RQ) && ok;
 #pragma unroll 2
       for (int a = 0; a < NQ; ++a)
         reinterpret_cast<double*>(line)[a] = fx::to_double(l.dot(tIt + a * S::RQ), l.x + l.kOut + xIt[a]);
     }
-    __syncthreads();
+    if (__syncthreads_or(!ok)) {
+      direct<NQ, CQ>(vg, cg, cubD, cubInterpT, offset, Ue, NUe, A, B, H);
+      continue;
+    }
     for (int n = tid; n < 3 * Np; n += S::THREADS) {
       const int ff = n / Np, m = n - ff * Np;
       NUe[ff * offset + m] = vg[kIJW * Np + m] * A[ff * AS + (m / (NQ * NQ)) * PS + (m / NQ % NQ) * LQ + m % NQ];
