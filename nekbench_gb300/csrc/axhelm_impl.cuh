@@ -55,35 +55,45 @@ struct Cfg {
 };
 
 // geometry of node (i,j,k) of an element from its trilinear coefficients
-// c[comp*8 + a], basis a = {1, r, s, t, rs, rt, st, rst}.
+// c[comp*8 + a], basis a = {1, r, s, t, rs, rt, st, rst}.  Every operation is the one of
+// trilinear_G2 (axhelm_l.cuh), so that an element's result is the same on small and on
+// large meshes.
 __device__ __forceinline__ void trilinear_G(const float* c, float r, float s, float t, float wijk,
                                             float& GwJ, float& G00, float& G01, float& G02,
                                             float& G11, float& G12, float& G22)
 {
+  const float rs = __fmul_rn(r, s), rt = __fmul_rn(r, t), st = __fmul_rn(s, t);
   float d[3][3];  // d[comp][dir]: x_r, x_s, x_t ...
 #pragma unroll
   for (int comp = 0; comp < 3; ++comp) {
     const float* a = c + comp * 8;
-    d[comp][0] = a[1] + a[4] * s + a[5] * t + a[7] * (s * t);
-    d[comp][1] = a[2] + a[4] * r + a[6] * t + a[7] * (r * t);
-    d[comp][2] = a[3] + a[5] * r + a[6] * s + a[7] * (r * s);
+    d[comp][0] = fmaf(a[7], st, fmaf(a[5], t, fmaf(a[4], s, a[1])));
+    d[comp][1] = fmaf(a[7], rt, fmaf(a[6], t, fmaf(a[4], r, a[2])));
+    d[comp][2] = fmaf(a[7], rs, fmaf(a[6], s, fmaf(a[5], r, a[3])));
   }
-  const float xr = d[0][0], xs = d[0][1], xt = d[0][2];
-  const float yr = d[1][0], ys = d[1][1], yt = d[1][2];
-  const float zr = d[2][0], zs = d[2][1], zt = d[2][2];
-  // cofactor rows: J * grad r, J * grad s, J * grad t
-  const float a0 = ys * zt - zs * yt, a1 = -(xs * zt - zs * xt), a2 = xs * yt - ys * xt;
-  const float b0 = -(yr * zt - zr * yt), b1 = xr * zt - zr * xt, b2 = -(xr * yt - yr * xt);
-  const float c0 = yr * zs - zr * ys, c1 = -(xr * zs - zr * xs), c2 = xr * ys - yr * xs;
-  const float J = xr * a0 + yr * a1 + zr * a2;
+  float cr[3][3];  // cr[dir][comp]: cofactors, J grad of the direction
+#pragma unroll
+  for (int dir = 0; dir < 3; ++dir) {
+    const int p = dir == 0 ? 1 : 0, q = dir == 2 ? 1 : 2;
+#pragma unroll
+    for (int comp = 0; comp < 3; ++comp) {
+      const int u = comp == 0 ? 1 : 0, v = comp == 2 ? 1 : 2;
+      cr[dir][comp] = (dir + comp) & 1 ? fmaf(-d[u][p], d[v][q], __fmul_rn(d[v][p], d[u][q]))
+                                       : fmaf(d[u][p], d[v][q], -__fmul_rn(d[v][p], d[u][q]));
+    }
+  }
+  const float J = fmaf(d[2][0], cr[0][2], fmaf(d[0][0], cr[0][0], __fmul_rn(d[1][0], cr[0][1])));
   const float winv = __fdividef(wijk, J);  // J > 0 and O(h^3): the fast divide is exact enough
-  GwJ = J * wijk;
-  G00 = winv * (a0 * a0 + a1 * a1 + a2 * a2);
-  G01 = winv * (a0 * b0 + a1 * b1 + a2 * b2);
-  G02 = winv * (a0 * c0 + a1 * c1 + a2 * c2);
-  G11 = winv * (b0 * b0 + b1 * b1 + b2 * b2);
-  G12 = winv * (b0 * c0 + b1 * c1 + b2 * c2);
-  G22 = winv * (c0 * c0 + c1 * c1 + c2 * c2);
+  auto dot = [&](int a, int b) {
+    return __fmul_rn(winv, fmaf(cr[a][2], cr[b][2], fmaf(cr[a][0], cr[b][0], __fmul_rn(cr[a][1], cr[b][1]))));
+  };
+  GwJ = __fmul_rn(J, wijk);
+  G00 = dot(0, 0);
+  G01 = dot(0, 1);
+  G02 = dot(0, 2);
+  G11 = dot(1, 1);
+  G12 = dot(1, 2);
+  G22 = dot(2, 2);
 }
 
 template <int NQ, int NF, bool BK, int PREC, bool DIR>  // DIR: q becomes the new direction z + beta q

@@ -15,8 +15,7 @@
 // of the CTA, without which the node passes wait for HBM (N=9, three fields: 500 against
 // 388 us in an early form).
 //
-// Every sum runs in the column form's order: the results are the same bits (FP32, BF16
-// storage; the trilinear geometry's divisions differ in the last place).  Even-odd
+// Every sum runs in the column form's order: the results are the same bits.  Even-odd
 // contractions were another 10 % faster but 7-11 % further from the exact result.
 //
 // Measured, 16.8 M nodes, column form -> this one (us): N=7 FP32 BK 110.7 -> 96.6 (6.3 TB/s),
@@ -175,7 +174,7 @@ __device__ __forceinline__ void column_dot(fw<W> (&t)[NQ], const float* tab)
   for (int p = 0; p < NQ; ++p) t[p] = row_dot<NQ, W>(tab, p, v);
 }
 
-// trilinear_G of two elements
+// trilinear_G (axhelm_impl.cuh) of two elements, operation for operation
 __device__ __forceinline__ void trilinear_G2(const f2* c, float r, float s, float t, float wijk, f2 (&G)[7])
 {
   const f2 r2 = pack(r, r), s2 = pack(s, s), t2 = pack(t, t), w2 = pack(wijk, wijk);
