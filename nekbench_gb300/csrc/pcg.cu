@@ -35,7 +35,10 @@ namespace nekb {
 namespace {
 
 constexpr int RT = 256;           // threads per reduction block
-constexpr int kMaxRedBlocks = 608;  // 152 SMs x 4: the FP64 sums of a block cost more than its waits
+// 152 SMs x 4 with vector access: the FP64 sums of a block cost more than its waits.  A thread
+// keeps a running sum per component of the vector, so its chains are no longer than those of
+// twice as many blocks with scalar access, which is what that takes.
+constexpr int kMaxRedBlocks = 608, kMaxRedBlocksScalar = 1216;
 
 enum { PC_COPY = 0, PC_JACOBI = 1, PC_EXTERNAL = 2 };
 
@@ -242,6 +245,15 @@ __device__ __forceinline__ void vst(T* p, const T (&v)[V])
   }
 }
 
+// sum of a thread's running sums, one per component
+template <int V, typename T>
+__device__ __forceinline__ T total(const T (&s)[V])
+{
+  if constexpr (V == 4) return (s[0] + s[1]) + (s[2] + s[3]);
+  if constexpr (V == 2) return s[0] + s[1];
+  return s[0];
+}
+
 // The passes over vectors keep their loops rolled: unrolled by four (the compiler's
 // choice) FP64 took 254 and not 233 us per iteration at E = 8192, N=7.
 //
@@ -252,7 +264,7 @@ __global__ void __launch_bounds__(RT) k_update_rz(PcgArgs<T> a)
   PcgState* st = a.st;
   if (st->done) return;
   const T alpha = UPDATE ? (T)st->alpha : T(0);
-  T rz = 0, rr = 0, za = 0;
+  T rz[V] = {}, rr[V] = {}, za[V] = {};
   const int64_t stride = (int64_t)gridDim.x * RT;
   const int64_t nv = a.Nloc / V;
   for (int f = 0; f < a.NF; ++f) {
@@ -290,17 +302,17 @@ __global__ void __launch_bounds__(RT) k_update_rz(PcgArgs<T> a)
       vld<V>(a.w + i, w);
 #pragma unroll
       for (int l = 0; l < V; ++l) {
-        if (MODE != PC_COPY) rz += w[l] * r[l] * z[l];  // else z = r: the same sum
-        rr += w[l] * r[l] * r[l];
-        if (FLEX) za += w[l] * z[l] * ap[l];
+        if (MODE != PC_COPY) rz[l] += w[l] * r[l] * z[l];  // else z = r: the same sum
+        rr[l] += w[l] * r[l] * r[l];
+        if (FLEX) za[l] += w[l] * z[l] * ap[l];
       }
     }
   }
   constexpr int NV = 1 + (MODE != PC_COPY) + FLEX;
   double v[NV];
-  v[0] = widen(rr);
-  if (MODE != PC_COPY) v[NV > 1 ? 1 : 0] = widen(rz);
-  if (FLEX) v[NV - 1] = widen(za);
+  v[0] = widen(total(rr));
+  if (MODE != PC_COPY) v[NV > 1 ? 1 : 0] = widen(total(rz));
+  if (FLEX) v[NV - 1] = widen(total(za));
   if (grid_sum<NV>(v, a.partials, a.counter)) {
     const double srz = MODE != PC_COPY ? v[NV > 1 ? 1 : 0] : v[0], sza = FLEX ? v[NV - 1] : 0.0;
     if (REFRESH)
@@ -354,7 +366,7 @@ __global__ void __launch_bounds__(RT) k_fcg_dots(PcgArgs<T> a, const T* __restri
   PcgState* st = a.st;
   if (st->done) return;
   const int cnt = st->fcg_count;
-  T rz = 0, rr = 0, zap[kFcgMax];
+  T rz[V] = {}, rr[V] = {}, zap[kFcgMax];
 #pragma unroll
   for (int j = 0; j < kFcgMax; ++j) zap[j] = 0;
   const int64_t stride = (int64_t)gridDim.x * RT;
@@ -370,23 +382,24 @@ __global__ void __launch_bounds__(RT) k_fcg_dots(PcgArgs<T> a, const T* __restri
       vld<V>(a.w + i, w);
 #pragma unroll
       for (int l = 0; l < V; ++l) {
-        rz += w[l] * r[l] * z[l];
-        rr += w[l] * r[l] * r[l];
+        rz[l] += w[l] * r[l] * z[l];
+        rr[l] += w[l] * r[l] * r[l];
       }
 #pragma unroll
       for (int j = 0; j < kFcgMax; ++j) {
         if (j < cnt) {
-          T ap[V];
+          T ap[V], sum = 0;  // of the vector first: a running sum per component would not fit the registers
           vld<V>(AP + j * ring + n, ap);
 #pragma unroll
-          for (int l = 0; l < V; ++l) zap[j] += w[l] * z[l] * ap[l];
+          for (int l = 0; l < V; ++l) sum += w[l] * z[l] * ap[l];
+          zap[j] += sum;
         }
       }
     }
   }
   double v[2 + kFcgMax];
-  v[0] = widen(rz);
-  v[1] = widen(rr);
+  v[0] = widen(total(rz));
+  v[1] = widen(total(rr));
 #pragma unroll
   for (int j = 0; j < kFcgMax; ++j) v[2 + j] = widen(zap[j]);
   if (grid_sum<2 + kFcgMax>(v, a.partials, a.counter)) {
@@ -437,7 +450,7 @@ __global__ void __launch_bounds__(RT) k_fcg_pap(PcgArgs<T> a, T* __restrict__ AP
   PcgState* st = a.st;
   if (st->done) return;
   const int head = st->fcg_head;
-  T pap = 0, rp = 0;
+  T pap[V] = {}, rp[V] = {};
   const int64_t stride = (int64_t)gridDim.x * RT;
   const int64_t nv = a.Nloc / V;
   for (int f = 0; f < a.NF; ++f) {
@@ -453,12 +466,12 @@ __global__ void __launch_bounds__(RT) k_fcg_pap(PcgArgs<T> a, T* __restrict__ AP
       vst<V>(AP + head * ring + n, ap);
 #pragma unroll
       for (int l = 0; l < V; ++l) {
-        pap += w[l] * p[l] * ap[l];
-        rp += w[l] * r[l] * p[l];
+        pap[l] += w[l] * p[l] * ap[l];
+        rp[l] += w[l] * r[l] * p[l];
       }
     }
   }
-  double v[2] = {widen(pap), widen(rp)};
+  double v[2] = {widen(total(pap)), widen(total(rp))};
   if (grid_sum<2>(v, a.partials, a.counter)) {
     const double pAp = v[0], alpha = v[1] / pAp;
     st->pAp = pAp;
@@ -481,7 +494,7 @@ __global__ void __launch_bounds__(RT) k_pap(PcgArgs<T> a)
 {
   PcgState* st = a.st;
   if (st->done) return;
-  T acc = 0;
+  T acc[V] = {};
   const int64_t stride = (int64_t)gridDim.x * RT;
   const int64_t nv = a.Nloc / V;
   for (int f = 0; f < a.NF; ++f) {
@@ -493,10 +506,10 @@ __global__ void __launch_bounds__(RT) k_pap(PcgArgs<T> a)
       vld<V>(a.p + iv * V + fo, p);
       vld<V>(a.Ap + iv * V + fo, ap);
 #pragma unroll
-      for (int l = 0; l < V; ++l) acc += w[l] * p[l] * ap[l];
+      for (int l = 0; l < V; ++l) acc[l] += w[l] * p[l] * ap[l];
     }
   }
-  double v[1] = {widen(acc)};
+  double v[1] = {widen(total(acc))};
   if (grid_sum<1>(v, a.partials, a.counter)) {
     const double pAp = v[0];
     const double alpha = st->rdotz1 / pAp;
@@ -601,11 +614,13 @@ __global__ void k_mask_set(int64_t Nm, const int32_t* ids, double v, double* q)
     q[ids[n]] = v;
 }
 
-inline unsigned red_grid(int64_t n)
+// blocks of a reduction over n entries, V to an access
+inline unsigned red_grid(int64_t n, int V)
 {
-  int64_t b = (n + RT - 1) / RT;
+  const int64_t most = V > 1 ? kMaxRedBlocks : kMaxRedBlocksScalar;
+  int64_t b = (n / V + RT - 1) / RT;
   if (b < 1) b = 1;
-  if (b > kMaxRedBlocks) b = kMaxRedBlocks;
+  if (b > most) b = most;
   return (unsigned)b;
 }
 
@@ -638,9 +653,9 @@ int launch_fcg_dots(const PcgArgs<T>& a, const ExtPrecond* ext, cudaStream_t s)
   if constexpr (sizeof(T) == 4) {
     const int64_t ring = a.NF * a.offset;
     if (a.Nloc % 4 == 0 && a.offset % 4 == 0)
-      k_fcg_dots<T, 4, REFRESH><<<red_grid(a.Nloc / 4), RT, 0, s>>>(a, ext->AP, ring);
+      k_fcg_dots<T, 4, REFRESH><<<red_grid(a.Nloc, 4), RT, 0, s>>>(a, ext->AP, ring);
     else
-      k_fcg_dots<T, 1, REFRESH><<<red_grid(a.Nloc), RT, 0, s>>>(a, ext->AP, ring);
+      k_fcg_dots<T, 1, REFRESH><<<red_grid(a.Nloc, 1), RT, 0, s>>>(a, ext->AP, ring);
     NEKB_CUDA(cudaGetLastError());
     return NEKB_OK;
   } else {
@@ -661,7 +676,7 @@ inline int vec_width(const PcgArgs<T>& a)
 template <typename T, int MODE, bool UPDATE, bool REFRESH, int V>
 void launch_rz_v(const PcgArgs<T>& a, bool flex, cudaStream_t s)
 {
-  const unsigned rg = red_grid(a.Nloc / V);
+  const unsigned rg = red_grid(a.Nloc, V);
   if (flex)
     k_update_rz<T, MODE, UPDATE, true, REFRESH, V><<<rg, RT, 0, s>>>(a);
   else
@@ -701,9 +716,9 @@ int launch_fcg_iteration(const OpView& op, PcgArgs<T> a, const ExtPrecond* ext, 
     NEKB_CUDA(cudaGetLastError());
     NEKB_TRY(apply_op(op, a.p, a.Ap, &a.st->done, s));
     if (v4) {
-      k_fcg_pap<T, 4><<<red_grid(a.Nloc / 4), RT, 0, s>>>(a, ext->AP, Nall);
+      k_fcg_pap<T, 4><<<red_grid(a.Nloc, 4), RT, 0, s>>>(a, ext->AP, Nall);
     } else {
-      k_fcg_pap<T, 1><<<red_grid(a.Nloc), RT, 0, s>>>(a, ext->AP, Nall);
+      k_fcg_pap<T, 1><<<red_grid(a.Nloc, 1), RT, 0, s>>>(a, ext->AP, Nall);
     }
     NEKB_CUDA(cudaGetLastError());
     if (net_takes_update(ext->net)) {  // x += alpha p, r -= alpha Ap inside the network kernel
@@ -753,7 +768,7 @@ int launch_iteration(const OpView& op, PcgArgs<T> a, int mode, bool flex, const 
   if (mode == PC_EXTERNAL && ext && ext->m > 1) return launch_fcg_iteration<T>(op, a, ext, s);
   const int64_t Nall = a.NF * a.offset;
   const int V = vec_width(a);
-  const unsigned vg = vec_grid(Nall / V), rg = red_grid(a.Nloc / V);
+  const unsigned vg = vec_grid(Nall / V), rg = red_grid(a.Nloc, V);
   constexpr int VW = sizeof(T) == 4 ? 4 : 2;
   if (sizeof(T) == 4 && ext && ext->axdot) {
     // FP32 operator: it takes the new direction on its way in and leaves the sums of p . A p,
@@ -812,7 +827,7 @@ int wdot(nekb_bp* bp, const T* w, const T* u, const T* v, int NF, double* result
   a.partials = bp->partials.as<double>();
   a.counter = bp->counter.as<unsigned>() + 4;
   a.out = bp->partials.as<double>() + 3 * 4096;
-  k_wdot<T, false><<<red_grid(a.Nloc), RT, 0, bp->stream>>>(a, u, v);
+  k_wdot<T, false><<<red_grid(a.Nloc, 1), RT, 0, bp->stream>>>(a, u, v);
   NEKB_CUDA(cudaGetLastError());
   NEKB_CUDA(cudaMemcpyAsync(result, a.out, sizeof(double), cudaMemcpyDeviceToHost, bp->stream));
   NEKB_CUDA(cudaStreamSynchronize(bp->stream));
@@ -1331,7 +1346,7 @@ int bp_zero_mean(nekb_bp* bp, double* q)
   const int64_t N = bp->E * (int64_t)bp->Np, Nall = bp->Nfields * bp->offset;
   if (N == 0) return NEKB_OK;
   double* out = bp->partials.as<double>() + 3 * 4096 + 4;
-  k_field_sum<<<red_grid(N), RT, 0, bp->stream>>>(N, bp->Nfields, bp->offset, q,
+  k_field_sum<<<red_grid(N, 1), RT, 0, bp->stream>>>(N, bp->Nfields, bp->offset, q,
                                                   bp->partials.as<double>(),
                                                   bp->counter.as<unsigned>() + 12, out);
   NEKB_CUDA(cudaGetLastError());
@@ -1354,7 +1369,7 @@ int bp_weighted_inner_product(nekb_bp* bp, const double* w, const double* a, con
   if (!bp || !w || !a || !b || !host_out) return fail(NEKB_ERR_INVALID, "weighted inner product: NULL argument");
   double* out = bp->partials.as<double>() + 3 * 4096;
   NEKB_TRY(launch_wdot(bp->Nlocal, bp->Nfields, bp->offset, w, a, b, two,
-                       red_grid(bp->Nlocal), bp->partials.as<double>(),
+                       red_grid(bp->Nlocal, 1), bp->partials.as<double>(),
                        bp->counter.as<unsigned>() + 8, out, bp->stream));
   NEKB_CUDA(cudaMemcpyAsync(host_out, out, sizeof(double) * (two ? 2 : 1), cudaMemcpyDeviceToHost, bp->stream));
   NEKB_CUDA(cudaStreamSynchronize(bp->stream));
