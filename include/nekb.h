@@ -50,9 +50,8 @@ extern "C" {
 #define NEKB_FP64_SPLIT      4  /* FP64 arrays as in NEKB_FP64, at low orders with arithmetic
                                    on the FP32 pipes in double-float form (~48 bits; agrees
                                    with NEKB_FP64 to ~1e-14 relative); |values| < 3.4e38; no
-                                   Partial forms.  From Nq = 8 (three fields: 5) on, and on
-                                   small and large meshes from Nq = 5 on, axhelm runs the
-                                   NEKB_FP64 operator, which is faster there                */
+                                   Partial forms.  From Nq = 5 on axhelm runs the NEKB_FP64
+                                   operator, which is faster on most meshes there           */
 
 /* gather-scatter data types and ops (3rdParty/ogs/ogs.hpp:128-140) */
 #define NEKB_DOUBLE 0

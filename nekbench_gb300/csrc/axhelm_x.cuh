@@ -291,10 +291,9 @@ int run_flags(int flags, const AxArgs& a, cudaStream_t s)
 {
   if (flags & NEKB_AX_PARTIAL)
     return fail(NEKB_ERR_UNSUPPORTED, "axhelm: Partial variants run in NEKB_FP64");
+  static_assert(NQ < kSplitFx, "NEKB_FP64_SPLIT runs the FP64 operator there");
   const bool bk = flags & NEKB_AX_BK;
-  if constexpr (NQ < kSplitFields3Fx) {  // above, three fields take the FP64 operator
-    if (flags & NEKB_AX_N3) return bk ? run<NQ, 3, true>(a, s) : run<NQ, 3, false>(a, s);
-  }
+  if (flags & NEKB_AX_N3) return bk ? run<NQ, 3, true>(a, s) : run<NQ, 3, false>(a, s);
   return bk ? run<NQ, 1, true>(a, s) : run<NQ, 1, false>(a, s);
 }
 

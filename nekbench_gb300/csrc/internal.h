@@ -67,9 +67,14 @@ __host__ __device__ constexpr int64_t line_nodes(int Nq, int fields, bool bk, in
   return 600000;
 }
 
-// The orders from which NEKB_FP64_SPLIT always runs the FP64 operator (axhelm_fx.cuh): one
-// field and three fields (launch_axhelm has the rule below them)
-constexpr int kSplitFx = 8, kSplitFields3Fx = 5;
+// The order from which NEKB_FP64_SPLIT runs the FP64 operator (axhelm_fx.cuh), which keeps more
+// digits and is the faster one there but for one field on meshes of medium size.  The rule does not
+// look at the mesh: an operator applied in parts has the bits of one call.  Double-float against
+// FP64, us: three fields N=3 307 / 361 (lambda, 2.5 M nodes), N=4 488 / 403.  One field, BK, by
+// elements: N=4 125 10.3 / 9.2, 1000 10.3 / 12.4, 110,592 380 / 375; N=5 512 12.4 / 10.3, 1331
+// 16.4 / 18.4, 64,000 402 / 386; N=6 576 16.4 / 14.4, 1000 20.5 / 26.6, 5832 88 / 72, 59,319
+// 803 / 596; N=7 167 / 123 (5.6 M nodes); N=11 283 / 171.
+constexpr int kSplitFx = 5;
 
 // ---------------------------------------------------------------- basis (host)
 int gll_nodes(int N, double* r, double* w);

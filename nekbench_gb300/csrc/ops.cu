@@ -30,9 +30,6 @@ NEKB_DECL_AX(tri)
 int launch_axhelm_x_nq2(int, const AxArgs&, cudaStream_t);
 int launch_axhelm_x_nq3(int, const AxArgs&, cudaStream_t);
 int launch_axhelm_x_nq4(int, const AxArgs&, cudaStream_t);
-int launch_axhelm_x_nq5(int, const AxArgs&, cudaStream_t);
-int launch_axhelm_x_nq6(int, const AxArgs&, cudaStream_t);
-int launch_axhelm_x_nq7(int, const AxArgs&, cudaStream_t);
 
 #define NEKB_SWITCH_AX(P)                                          \
   switch (Nq) {                                                    \
@@ -50,21 +47,6 @@ int launch_axhelm_x_nq7(int, const AxArgs&, cudaStream_t);
   }                                                                \
   break;
 
-// Whether NEKB_FP64_SPLIT runs the FP64 operator, which keeps more digits and is the faster
-// one but at the lowest orders and, at Nq = 5 to 7, on meshes of medium size.  Double-float
-// against FP64, us: three fields N=3 307 / 361 (lambda, 2.5 M nodes), N=4 488 / 403; N=7 167 / 123
-// (5.6 M nodes); N=11 283 / 171.  One field, BK, by elements: N=4 125 10.3 / 9.2, 729 10.4 / 10.4,
-// 1000 10.3 / 12.4, 31,744 116 / 121, 64,000 224 / 223, 110,592 380 / 375; N=5 512 12.4 / 10.3,
-// 1331 16.4 / 18.4, 14,400 97 / 98, 64,000 402 / 386; N=6 576 16.4 / 14.4, 1000 20.5 / 26.6,
-// 4096 60.2 / 59.1, 5832 88 / 72, 59,319 803 / 596; with lambda FP64 is ahead by up to 15 % more.
-static bool split_runs_fp64(int Nq, bool three, int64_t E)
-{
-  if (Nq >= (three ? kSplitFields3Fx : kSplitFx)) return true;
-  if (three || Nq < 5) return false;
-  const int64_t lines = E * Nq * Nq;
-  return lines <= 152 * 120 || lines * Nq >= (Nq == 7 ? 2000000 : 8000000);
-}
-
 int launch_axhelm(int Nq, int flags, int precision, const AxArgs& a, cudaStream_t s)
 {
   if (Nq < kMinNq || Nq > kMaxNq) return fail(NEKB_ERR_UNSUPPORTED, "axhelm: Nq=%d outside 2..%d", Nq, kMaxNq);
@@ -76,7 +58,7 @@ int launch_axhelm(int Nq, int flags, int precision, const AxArgs& a, cudaStream_
   if (precision == NEKB_FP64_SPLIT) {
     if (flags & NEKB_AX_PARTIAL)
       return fail(NEKB_ERR_UNSUPPORTED, "axhelm: Partial variants run in NEKB_FP64");
-    if (split_runs_fp64(Nq, flags & NEKB_AX_N3, a.Nelements)) precision = NEKB_FP64;
+    if (Nq >= kSplitFx) precision = NEKB_FP64;
   }
   if (precision == NEKB_FP64 && Nq == 13) return launch_axhelm_f64_nq13(flags, a, s);
   if (precision == NEKB_FP64 && Nq == 14) return launch_axhelm_f64_nq14(flags, a, s);
@@ -90,9 +72,6 @@ int launch_axhelm(int Nq, int flags, int precision, const AxArgs& a, cudaStream_
         case 2: return launch_axhelm_x_nq2(flags, a, s);
         case 3: return launch_axhelm_x_nq3(flags, a, s);
         case 4: return launch_axhelm_x_nq4(flags, a, s);
-        case 5: return launch_axhelm_x_nq5(flags, a, s);
-        case 6: return launch_axhelm_x_nq6(flags, a, s);
-        case 7: return launch_axhelm_x_nq7(flags, a, s);
       }
       break;
     default: break;

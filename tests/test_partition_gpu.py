@@ -75,3 +75,16 @@ def test_fp32_forms_by_lines_and_by_columns(nb, O, dev, N, flags, form):
         g, per = T(m.ggeo, dev, torch.bfloat16 if prec == nb.BF16 else F), 7 * Np
     lam = None if flags & nb.AX_BK else T(lam, dev, torch.bfloat16 if prec == nb.BF16 else F)
     whole_and_chunks(nb, N, E, flags, prec, per, g, T(m.D, dev, F), lam, T(q, dev, F), [1, E // 3, E // 2])
+
+
+@pytest.mark.parametrize("N,E", [(1, 700), (3, 800), (4, 2400), (5, 1400), (6, 6000), (7, 1600), (8, 650), (13, 300)])
+@pytest.mark.parametrize("flags", [0, 3])
+@pytest.mark.parametrize("form", ["FP64", "FP64_SPLIT"])
+def test_fp64_forms(nb, O, dev, N, E, flags, form):
+    """Across the line between three groups of threads per element and one (FP64)."""
+    if form == "FP64_SPLIT" and N > 11:
+        pytest.skip("built for N <= 11")
+    m, lam, q = problem(O, N, E, 3 if flags & nb.AX_N3 else 1)
+    lam = None if flags & nb.AX_BK else T(lam, dev)
+    whole_and_chunks(nb, N, E, flags, getattr(nb, form), 7 * (N + 1) ** 3, T(m.ggeo, dev), T(m.D, dev), lam, T(q, dev),
+                     [2, E // 8, E // 2])
