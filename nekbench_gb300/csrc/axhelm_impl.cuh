@@ -96,6 +96,14 @@ __device__ __forceinline__ void trilinear_G(const float* c, float r, float s, fl
   G22 = dot(2, 2);
 }
 
+// whether the solve is over; the block sums' reader learns it from their count
+__device__ __forceinline__ bool skipped(const AxArgs& a)
+{
+  if (a.skip == nullptr || *a.skip == 0) return false;
+  if (a.dot_count != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *a.dot_count = 0;
+  return true;
+}
+
 template <int NQ, int NF, bool BK, int PREC, bool DIR>  // DIR: q becomes the new direction z + beta q
 __global__ void __launch_bounds__(Cfg<NQ, NF, PREC>::THREADS, Cfg<NQ, NF, PREC>::MINB)
 k_axhelm(const AxArgs a)
@@ -104,7 +112,7 @@ k_axhelm(const AxArgs a)
   using T = typename Prec<PREC>::T;
   using TG = typename Prec<PREC>::TG;
   constexpr int NQ2 = C::NQ2, NP = C::NP, NEL = C::NEL, DS = NQ + 1;
-  if (a.skip != nullptr && *a.skip != 0) return;
+  if (skipped(a)) return;
 
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* s_D = reinterpret_cast<T*>(smem_raw);

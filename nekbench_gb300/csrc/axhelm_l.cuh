@@ -224,7 +224,7 @@ k_axhelm_l(const AxArgs a)
   constexpr int W = NF;
   constexpr int NQ2 = C::NQ2, NP = C::NP, LS = C::LS, PS = C::PS, AS = C::AS;
   using V = fw<W>;
-  if (a.skip != nullptr && *a.skip != 0) return;
+  if (skipped(a)) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   float* s_D = reinterpret_cast<float*>(smem_raw);
   float* s_Dt = s_D + C::TAB;

@@ -107,7 +107,8 @@ struct AxArgs {
   void* Aq;
   const int* skip;      // optional device flag: kernel returns at once when *skip != 0
   // optional: per-block sums of q . Aq (local, before assembly) into
-  // dot_partials[block], the block count into *dot_count (non-Partial forms)
+  // dot_partials[block], the block count into *dot_count (non-Partial forms; 0 where the
+  // operator is skipped)
   double* dot_partials;
   int* dot_count;
   // optional (4-byte vectors): q is first replaced by z + (float)*beta q, the conjugate

@@ -315,7 +315,9 @@ template <typename T>
 __global__ void __launch_bounds__(kGsThreads) k_gs_add(GsGroups g, int k, int64_t stride, T* __restrict__ q,
                                                        const int* skip, GsExtra x)
 {
-  if (skip != nullptr && *skip != 0) return;
+  // With st this launch may set the flag that skip points to, so it looks at what the operator
+  // before it left instead.
+  if (x.st != nullptr ? *x.count == 0 : skip != nullptr && *skip != 0) return;
   const int tid = threadIdx.x;
   constexpr int kStep = kGsThreads;
   if ((int)blockIdx.x < x.first) {
