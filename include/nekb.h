@@ -319,6 +319,10 @@ int nekb_adv_cubature(int Nq, int cubNq, int precision, int64_t Nelements, const
 void nekb_pcg_default_opts(nekb_pcg_opts* opts);
 int nekb_bp_pcg(nekb_bp* bp, const double* lambda, double* r, double* x, double tol, int maxit,
                 const nekb_pcg_opts* opts, nekb_pcg_stats* stats);
+/* How often a kernel of this process was prepared (shared-memory opt-in) inside one of the
+ * solvers' graph captures; 0, as every kernel of an iteration is prepared by a launch before
+ * the capture.  For a test of that.  No counterpart in the reference. */
+int nekb_captured_opt_ins(void);
 
 /* ------------------------------------------------------------------ learned preconditioner
  * Per-element 3D convolution network: layers of 3x3x3 convolutions on the Nq^3

@@ -47,7 +47,7 @@ EXPORTED = [
     "nekb_net_num_params", "nekb_net_get_weights",
     "nekb_net_set_weights", "nekb_net_forward", "nekb_net_raise_copy_timeout", "nekb_net_train_step", "nekb_net_gradient",
     "nekb_net_prepare_pairs", "nekb_net_save", "nekb_net_load", "nekb_peak_fma", "nekb_peak_copy",
-    "nekb_dot_num_blocks", "nekb_dot_partials", "nekb_adv_cubature",
+    "nekb_dot_num_blocks", "nekb_dot_partials", "nekb_adv_cubature", "nekb_captured_opt_ins",
 ]
 
 

@@ -326,26 +326,30 @@ k_axhelm(const AxArgs a)
 
 // A kernel of its own for the direction update: as a branch in the plain operator it cost that
 // 2 to 6 % at N=1 and 2 (16.2 M elements, N=1 BK: FP32 839 against 816 us, BF16 721 / 685).
-template <int NQ, int NF, bool BK, int PREC, bool DIR>
+// Built for one field only: with three the solver updates the direction apart (pcg.cu).
+template <int NQ, int NF, bool BK, int PREC>
 int run(const AxArgs& a, cudaStream_t s)
 {
   using C = Cfg<NQ, NF, PREC>;
-  auto kern = k_axhelm<NQ, NF, BK, PREC, DIR>;
-  // opt in to >48 KB of shared memory at the first launch on each device
+  auto kern = k_axhelm<NQ, NF, BK, PREC, false>;
+  // opt in to >48 KB of shared memory (dynamic + static may pass that) at the first launch on
+  // each device, of both kernels: the solvers launch the plain one before a capture that
+  // holds the other
   static SmemOptIn smem_opt;
-  NEKB_TRY(smem_opt.ensure(kern, C::SMEM));  // dynamic + static may pass 48 KB
+  NEKB_TRY(smem_opt.ensure(kern, C::SMEM));
+  if constexpr (NF == 1) {
+    static SmemOptIn smem_dir;
+    NEKB_TRY(smem_dir.ensure(k_axhelm<NQ, NF, BK, PREC, true>, C::SMEM));
+    if (a.z != nullptr) kern = k_axhelm<NQ, NF, BK, PREC, true>;
+  } else if (a.z != nullptr) {
+    return fail(NEKB_ERR_UNSUPPORTED, "axhelm: direction update of three fields");
+  }
   const int64_t nblk = (a.Nelements + C::NEL - 1) / C::NEL;
   if (nblk == 0) return NEKB_OK;
   if (nblk > INT_MAX) return fail(NEKB_ERR_INVALID, "axhelm: too many elements");
   kern<<<(unsigned)nblk, C::THREADS, C::SMEM, s>>>(a);
   NEKB_CUDA(cudaGetLastError());
   return NEKB_OK;
-}
-
-template <int NQ, int NF, bool BK, int PREC>
-int run(const AxArgs& a, cudaStream_t s)
-{
-  return a.z != nullptr ? run<NQ, NF, BK, PREC, true>(a, s) : run<NQ, NF, BK, PREC, false>(a, s);
 }
 
 }  // namespace ax

@@ -29,6 +29,8 @@ int bp_zero_mean(nekb_bp* bp, double* q);
 
 using namespace nekb;
 
+extern "C" int nekb_captured_opt_ins(void) { return g_captured_opt_ins.load(); }
+
 namespace {
 // GLL nodes/weights per order, for the trilinear-geometry operator
 struct NodeCache {

@@ -14,6 +14,8 @@ namespace nekb {
 
 // ------------------------------------------------------------------ errors
 static thread_local char g_err[512] = "";
+thread_local bool t_capturing = false;
+std::atomic<int> g_captured_opt_ins{0};
 
 int fail(int code, const char* fmt, ...)
 {

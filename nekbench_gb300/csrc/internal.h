@@ -33,7 +33,10 @@ void clear_error();
 // attribute belongs to each device's context, so it is set once per device
 // (ordinals 0..63 are remembered; beyond that it is set at every launch).  The
 // solvers launch every operator once before they capture a graph, so the
-// first launch on a device never falls inside a capture.
+// first launch on a device never falls inside a capture (g_captured_opt_ins counts
+// those that do).
+extern thread_local bool t_capturing;        // this thread is in one of the solvers' captures
+extern std::atomic<int> g_captured_opt_ins;
 struct SmemOptIn {
   std::atomic<uint64_t> done{0};
   template <typename K>
@@ -43,6 +46,7 @@ struct SmemOptIn {
     NEKB_CUDA(cudaGetDevice(&dev));
     const uint64_t bit = (dev >= 0 && dev < 64) ? (uint64_t(1) << dev) : 0;
     if (bit != 0 && (done.load(std::memory_order_acquire) & bit) != 0) return 0;
+    if (t_capturing) ++g_captured_opt_ins;
     NEKB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
     done.fetch_or(bit, std::memory_order_release);
     return 0;

@@ -561,12 +561,11 @@ int net_infer_tc5(const __nv_bfloat16* Wbf, int64_t Etot, int64_t Efield, const 
                   const float* invDiag, float* out, int normalize, const int* skip, cudaStream_t s,
                   const NetUpdate* up)
 {
+  // both at the first launch of either: the solver launches the plain kernel before it captures
+  // an iteration with the other
   static SmemOptIn smem_plain, smem_update;
-  if (up) {
-    NEKB_TRY(smem_update.ensure(k_net_infer_tc5<true>, kSmTotal));
-  } else {
-    NEKB_TRY(smem_plain.ensure(k_net_infer_tc5<false>, kSmTotal));
-  }
+  NEKB_TRY(smem_plain.ensure(k_net_infer_tc5<false>, kSmTotal));
+  NEKB_TRY(smem_update.ensure(k_net_infer_tc5<true>, kSmTotal));
   int dev = 0, sms = 152;
   NEKB_CUDA(cudaGetDevice(&dev));
   NEKB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));

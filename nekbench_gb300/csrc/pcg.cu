@@ -920,8 +920,10 @@ int pcg_core(nekb_bp* bp, const OpView& op, T* r, T* x, const T* w, const T* inv
       cudaGraph_t g = nullptr;
       NEKB_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
       int st_cap = NEKB_OK;
+      t_capturing = true;
       for (int c = 0; c < chunk && st_cap == NEKB_OK; ++c)
         st_cap = launch_iteration<T>(op, a, mode, flex, ext, s);
+      t_capturing = false;
       cudaError_t ce = cudaStreamEndCapture(s, &g);
       if (st_cap != NEKB_OK) {
         if (g) cudaGraphDestroy(g);
