@@ -26,6 +26,7 @@
 #include "bp.h"
 #include "nn.h"
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <functional>
@@ -39,6 +40,10 @@ constexpr int RT = 256;           // threads per reduction block
 // keeps a running sum per component of the vector, so its chains are no longer than those of
 // twice as many blocks with scalar access, which is what that takes.
 constexpr int kMaxRedBlocks = 608, kMaxRedBlocksScalar = 1216;
+// k_fcg_dots has ten sums per block: two blocks per SM, each thread with up to eleven loads in
+// flight (N=7, 13,824 elements, us per iteration of the learned solve: 606, with 608 blocks of 64
+// registers 622, of 99 registers 620); the chains are those of 1216 blocks with scalar access
+constexpr int kFcgDotsBlocks = 304;
 
 enum { PC_COPY = 0, PC_JACOBI = 1, PC_EXTERNAL = 2 };
 
@@ -361,7 +366,7 @@ __global__ void __launch_bounds__(RT) k_pupdate(PcgArgs<T> a)
 
 // (r, z) sums and z . A p_j for the kept directions; REFRESH: same iteration
 template <typename T, int V, bool REFRESH>
-__global__ void __launch_bounds__(RT) k_fcg_dots(PcgArgs<T> a, const T* __restrict__ AP, int64_t ring)
+__global__ void __launch_bounds__(RT, 2) k_fcg_dots(PcgArgs<T> a, const T* __restrict__ AP, int64_t ring)
 {
   PcgState* st = a.st;
   if (st->done) return;
@@ -376,10 +381,13 @@ __global__ void __launch_bounds__(RT) k_fcg_dots(PcgArgs<T> a, const T* __restri
 #pragma unroll 1
     for (int64_t iv = (int64_t)blockIdx.x * RT + threadIdx.x; iv < nv; iv += stride) {
       const int64_t i = iv * V, n = i + fo;
-      T r[V], z[V], w[V];
+      T r[V], z[V], w[V], ap[kFcgMax][V];
       vld<V>(a.r + n, r);
       vld<V>(a.z + n, z);
       vld<V>(a.w + i, w);
+#pragma unroll
+      for (int j = 0; j < kFcgMax; ++j)
+        if (j < cnt) vld<V>(AP + j * ring + n, ap[j]);
 #pragma unroll
       for (int l = 0; l < V; ++l) {
         rz[l] += w[l] * r[l] * z[l];
@@ -388,10 +396,9 @@ __global__ void __launch_bounds__(RT) k_fcg_dots(PcgArgs<T> a, const T* __restri
 #pragma unroll
       for (int j = 0; j < kFcgMax; ++j) {
         if (j < cnt) {
-          T ap[V], sum = 0;  // of the vector first: a running sum per component would not fit the registers
-          vld<V>(AP + j * ring + n, ap);
+          T sum = 0;  // of the vector first: a running sum per component would take 32 registers
 #pragma unroll
-          for (int l = 0; l < V; ++l) sum += w[l] * z[l] * ap[l];
+          for (int l = 0; l < V; ++l) sum += w[l] * z[l] * ap[j][l];
           zap[j] += sum;
         }
       }
@@ -653,7 +660,7 @@ int launch_fcg_dots(const PcgArgs<T>& a, const ExtPrecond* ext, cudaStream_t s)
   if constexpr (sizeof(T) == 4) {
     const int64_t ring = a.NF * a.offset;
     if (a.Nloc % 4 == 0 && a.offset % 4 == 0)
-      k_fcg_dots<T, 4, REFRESH><<<red_grid(a.Nloc, 4), RT, 0, s>>>(a, ext->AP, ring);
+      k_fcg_dots<T, 4, REFRESH><<<std::min<unsigned>(red_grid(a.Nloc, 4), kFcgDotsBlocks), RT, 0, s>>>(a, ext->AP, ring);
     else
       k_fcg_dots<T, 1, REFRESH><<<red_grid(a.Nloc, 1), RT, 0, s>>>(a, ext->AP, ring);
     NEKB_CUDA(cudaGetLastError());
