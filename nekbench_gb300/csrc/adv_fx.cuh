@@ -17,21 +17,22 @@
 // registers; H holds the contravariant velocity.  Everything before and after is
 // overlaid on them.
 //
-// E = 8192, N=7, cubN=11: FP64 FMAs 6.06 ms, double-float 3.80, this 2.94 (the integer
-// multiply-add pipe 47 % busy, FP64 17 %; one CTA per SM, whose passes alternate between
-// the two); N=7, cubN=7: 1.67, 1.05, 0.77; N=2, cubN=2, 155,344 elements: 2.70, 1.60, 0.56.
-// Requesting the next element's metric terms into L2 and unrolling the pointwise passes
-// changed nothing.
+// E = 8192, us: N=7, cubN=11 FP64 FMAs 6060, double-float 3800, this 2966 (the integer multiply-add
+// pipe 35 % busy, FP64 17 %; one CTA per SM, whose passes alternate between the two); Gauss
+// nodes, N=7, cubN=7 792; the element's own nodes 1670, 1050, 334; N=2, cubN=2, 155,344 elements, own
+// nodes 2700, 1600, 310.  Requesting the next element's metric terms into L2 and unrolling the
+// pointwise passes changed nothing.
 //
 // An element with values that have no fixed-point form, and all elements when a matrix
 // has none, are evaluated with FP64 sums (direct).  A line shares one exponent, so where a
 // zero of a matrix meets a value far above the others the result would be short of bits
-// (fixedpt.cuh).  The node that odd Gauss and Gauss-Lobatto grids share, the centre, has such
-// zeros in the interpolation beside it and in the derivative on the diagonal: an element with
-// a line to be derived or projected that has too small terms there takes the FP64 sums too.
-// So do all elements when zeros stand in more than one row, as when the cubature nodes are the
-// element's own (the interpolation is then the identity, and every value small beside its
-// line's largest would lose).
+// (fixedpt.cuh).  Nodes that the cubature grid shares with the element's (the centre, and the
+// ends of Gauss-Lobatto grids) are such places: their rows of the interpolation have one entry,
+// and the derivative has zeros on its diagonal.  An element with a line to be derived or
+// projected that has too small terms there takes the FP64 sums too; an interpolated value short
+// of bits is one term among larger ones of the projection, as long as some row is full.
+// Where the grids are the same, the interpolation is the identity, no row is full and every
+// value counts: then U is taken as it is, and the advection terms are the result.
 #pragma once
 #include "adv_impl.cuh"
 #include "fixedpt.cuh"
@@ -59,7 +60,7 @@ struct Shape {
   static constexpr int LN = NQ | 1;
   static constexpr int RN = (NQ + 1) & ~1, RQ = (CQ + 1) & ~1;   // table rows of NQ and of CQ entries
   static constexpr int TAB = CQ * RN + NQ * RQ + CQ * RQ;        // I, I^T, D
-  static constexpr int EXPS = 3 * 3 * CQ2 + 2 * CQ + NQ;
+  static constexpr int EXPS = 3 * 3 * CQ2 + 2 * CQ + NQ + 2;  // and the matrices' rows with zeros
   static constexpr int SMEM = (TAB + 9 * AS) * 8 + EXPS * 4;
   // CTAs per SM: as many as shared memory holds and registers of this number.  More CTAs
   // beat fewer spills, most on small grids (500,000 nodes, us at 128 / 80 / 64 registers: N=2,
@@ -83,8 +84,23 @@ struct Ln : fx::Line<N, false> {
     x = this->e - 1075 - F::kVUp;
     return ok && (this->e == 200 || (this->e >= lo && this->e <= hi));
   }
-  // from results r[m] 2^e[m] (each standing for r + 1/2): normalised, aligned, rounded
-  __device__ __forceinline__ void from(const long long (&r)[N], const int (&e)[N])
+  // the same for a line to be projected: gap is to the largest of the entries in full rows
+  __device__ __forceinline__ bool from(const double (&v)[N], int lo, int hi, unsigned full)
+  {
+    const bool ok = from(v, lo, hi);
+    unsigned top = 0, next = 0;
+#pragma unroll
+    for (int a = 0; a < N; ++a) {
+      top = max(top, fx::hi_abs(v[a]));
+      if (full >> a & 1u) next = max(next, fx::hi_abs(v[a]));
+    }
+    this->gap = next != 0u ? top - next : 0u;
+    return ok;
+  }
+  // from results r[m] 2^e[m] (each standing for r + 1/2): normalised, aligned, rounded; PROJECT:
+  // gap to the entries in full rows, else to the second largest
+  template <bool PROJECT = false>
+  __device__ __forceinline__ void from(const long long (&r)[N], const int (&e)[N], unsigned full = 0)
   {
     long long m[N];
     int ex[N], top = -100000, second = -100000;
@@ -94,7 +110,10 @@ struct Ln : fx::Line<N, false> {
       ex[a] = lz == 64 ? -100000 : e[a] - (lz - 1);
       m[a] = lz == 64 ? 0 : r[a];
       asm("shl.b64 %0, %0, %1;" : "+l"(m[a]) : "r"(lz - 1));
-      if (N > 2) second = max(second, min(top, ex[a]));
+      if (PROJECT)
+        second = full >> a & 1u ? max(second, ex[a]) : second;
+      else if (N > 2)
+        second = max(second, min(top, ex[a]));
       top = max(top, ex[a]);
     }
     constexpr int down = 10 - F::kVUp;  // 63-bit magnitudes to 53 + kVUp bits
@@ -117,29 +136,34 @@ struct Ln : fx::Line<N, false> {
 };
 
 // Rows (stride RS) of a matrix of ROWS x COLS entries at M[p ps + m ms], with the exponents
-// of their entries (value = entry 2^ex) in ex; whether the matrix has a fixed-point form, in
-// every thread: every row in range, and, with COUNT, zeros (kZero; DIAG: beside the diagonal)
-// in one row at most (two columns: none).  The block synchronises here.
-template <int ROWS, int COLS, int RS, bool COUNT, bool DIAG = false>
-__device__ __forceinline__ bool fill(const double* __restrict__ M, int ps, int ms, int2* t, int* ex)
+// of their entries (value = entry 2^ex) in ex; whether every row has a fixed-point form, in
+// every thread.  rows, if given: bit p is set for a row with zeros (kZero; DIAG: beside the
+// diagonal; two columns: anywhere), bit 31 if every row is the identity's.  The block synchronises here.
+template <int ROWS, int COLS, int RS, bool DIAG = false>
+__device__ __forceinline__ bool fill(const double* __restrict__ M, int ps, int ms, int2* t, int* ex,
+                                     unsigned* rows = nullptr)
 {
-  static_assert(ROWS <= 32, "one row per thread");
-  bool ok = true, zeros = false;
+  static_assert(ROWS <= 31, "one row per thread of a warp");
+  bool ok = true, zeros = false, unit = true;
   if (threadIdx.x < ROWS) {
     const int p = threadIdx.x;
     unsigned mx = 0, least = 0x7fffffffu;
     for (int m = 0; m < COLS; ++m) {
-      const unsigned v = fx::hi_abs(M[p * ps + m * ms]);
-      mx = max(mx, v);
-      if (!DIAG || COLS == 2 || m != p) least = min(least, v);
+      const double v = M[p * ps + m * ms];
+      mx = max(mx, fx::hi_abs(v));
+      if (!DIAG || COLS == 2 || m != p) least = min(least, fx::hi_abs(v));
+      unit = unit && v == (m == p ? 1.0 : 0.0);
     }
     const int e = (int)(mx >> 20);
     ok = e >= kMLo && e <= kMHi;
     zeros = least + ((unsigned)kZero << 20) < mx;
     ex[p] = e;
   }
-  bool all = !__syncthreads_or(!ok);
-  if (COUNT) all = __syncthreads_count(zeros) <= (COLS == 2 ? 0 : 1) && all;
+  if (rows != nullptr && threadIdx.x < 32) {
+    const unsigned z = __ballot_sync(0xffffffffu, zeros), u = __all_sync(0xffffffffu, unit);
+    if (threadIdx.x == 0) *rows = z | (u && ROWS == COLS ? 1u << 31 : 0u);
+  }
+  const bool all = !__syncthreads_or(!ok);
   for (int n = threadIdx.x; n < ROWS * RS; n += blockDim.x) {
     const int p = n / RS, m = n - p * RS;
     int2 w = make_int2(0, 0);
@@ -254,22 +278,22 @@ k_adv_fx(int64_t E, const double* __restrict__ vgeo, const double* __restrict__ 
   long long* Hi = reinterpret_cast<long long*>(H);
 
   const int tid = threadIdx.x;
-  bool m_ok = fill<CQ, NQ, S::RN, true>(cubInterpT, 1, CQ, tI, xI);
-  m_ok = fill<NQ, CQ, S::RQ, false>(cubInterpT, CQ, 1, tIt, xIt) && m_ok;
-  m_ok = fill<CQ, CQ, S::RQ, true, true>(cubD, CQ, 1, tD, xD) && m_ok;
+  unsigned* rows = reinterpret_cast<unsigned*>(xD + CQ);
+  bool m_ok = fill<CQ, NQ, S::RN>(cubInterpT, 1, CQ, tI, xI, rows);
+  m_ok = fill<NQ, CQ, S::RQ>(cubInterpT, CQ, 1, tIt, xIt) && m_ok;
+  m_ok = fill<CQ, CQ, S::RQ, true>(cubD, CQ, 1, tD, xD, rows + 1) && m_ok;
+  const bool same = NQ == CQ && rows[0] >> 31;  // the cubature nodes are the element's own
+  const unsigned full = ~rows[0] & ((1u << CQ) - 1u);  // full rows of the interpolation
+  m_ok = m_ok && (same || full != 0u) && __popc(rows[1] & 0x7fffffffu) <= (CQ == 2 ? 0 : 1);
 
   // the thread's component and column (i, j); also the numbers of its lines
   const bool act = tid < 3 * CQ2;
   const int f = act ? tid / CQ2 : 0, ij = act ? tid - f * CQ2 : 0, i = ij % CQ, j = ij / CQ;
   const int col = f * AS + j * LQ + i;
 
-  for (int64_t e = blockIdx.x; e < E; e += gridDim.x) {
-    const double* Ue = U + e * Np;
-    const double* cg = cubvgeo + e * (int64_t)Cp * kNvgeo;
-    const double* vg = vgeo + e * (int64_t)Np * kNvgeo;
-    double* NUe = NU + e * Np;
-    bool ok = m_ok;
-    __syncthreads();  // exponents written; the previous element's last reads
+  // cubature values: A and B [f][k][j][i], exponent e3[(f,j,i)] + xI[k]; whether U has a fixed-point form
+  auto interpolate = [&](const double* Ue) {
+    bool ok = true;
     for (int n = tid; n < 3 * Np; n += S::THREADS) {
       const int ff = n / Np, m = n - ff * Np;
       A[(n / NQ) * LN + n % NQ] = Ue[ff * offset + m];
@@ -304,7 +328,7 @@ k_adv_fx(int64_t E, const double* __restrict__ vgeo, const double* __restrict__ 
       for (int p = 0; p < CQ; ++p) Hi[(fc * CQ + p) * LQ + ii] = l.dot(tI + p * S::RN);
     }
     __syncthreads();
-    // in t: line (f,j,i) -> A and B [f][k][j][i], exponent e3[(f,j,i)] + xI[k]
+    // in t: line (f,j,i) -> A and B
     if (act) {
       long long r[NQ];
       int x[NQ];
@@ -323,18 +347,43 @@ k_adv_fx(int64_t E, const double* __restrict__ vgeo, const double* __restrict__ 
         Bi[col + p * PS] = v;
       }
     }
+    return ok;
+  };
+
+  for (int64_t e = blockIdx.x; e < E; e += gridDim.x) {
+    const double* Ue = U + e * Np;
+    const double* cg = cubvgeo + e * (int64_t)Cp * kNvgeo;
+    const double* vg = vgeo + e * (int64_t)Np * kNvgeo;
+    double* NUe = NU + e * Np;
+    bool ok = m_ok;
+    __syncthreads();  // exponents written; the previous element's last reads
+    if (same) {  // cubature values are U: A and B [f][k][j][i] as FP64
+      for (int n = tid; n < 3 * Np; n += S::THREADS) {
+        const int ff = n / Np, m = n - ff * Np, at = ff * AS + (m / (NQ * NQ)) * PS + (m / NQ % NQ) * LQ + m % NQ;
+        A[at] = B[at] = Ue[ff * offset + m];
+      }
+    } else {
+      ok = interpolate(Ue) && ok;
+    }
     __syncthreads();
     // contravariant velocity into H, a third of the planes per group; the column for the t derivative
     Ln<CQ> t;
     if (act) {
-      long long r[CQ];
-      int x[CQ];
+      if (same) {
+        double v[CQ];
 #pragma unroll
-      for (int k = 0; k < CQ; ++k) {
-        r[k] = Ai[col + k * PS];
-        x[k] = e3[tid] + xI[k];
+        for (int k = 0; k < CQ; ++k) v[k] = A[col + k * PS];
+        ok = t.from(v, kULo, kUHi) && ok;
+      } else {
+        long long r[CQ];
+        int x[CQ];
+#pragma unroll
+        for (int k = 0; k < CQ; ++k) {
+          r[k] = Ai[col + k * PS];
+          x[k] = e3[tid] + xI[k];
+        }
+        t.from(r, x);
       }
-      t.from(r, x);
       ok = t.fits(tD, CQ, S::RQ) && ok;
 #pragma unroll 1
       for (int k = f; k < CQ; k += 3) {
@@ -342,7 +391,8 @@ k_adv_fx(int64_t E, const double* __restrict__ vgeo, const double* __restrict__ 
         const double* g = cg + k * CQ2 + ij;
         double u[3];
 #pragma unroll
-        for (int ff = 0; ff < 3; ++ff) u[ff] = fx::to_double(Ai[ff * AS + n], e3[ff * CQ2 + ij] + xI[k]);
+        for (int ff = 0; ff < 3; ++ff)
+          u[ff] = same ? A[ff * AS + n] : fx::to_double(Ai[ff * AS + n], e3[ff * CQ2 + ij] + xI[k]);
         const double JW = g[kJW * Cp];
         H[n] = JW * fma(u[2], g[kRZ * Cp], fma(u[1], g[kRY * Cp], u[0] * g[kRX * Cp]));
         H[AS + n] = JW * fma(u[2], g[kSZ * Cp], fma(u[1], g[kSY * Cp], u[0] * g[kSX * Cp]));
@@ -350,33 +400,33 @@ k_adv_fx(int64_t E, const double* __restrict__ vgeo, const double* __restrict__ 
       }
     }
     __syncthreads();
-    // derivatives in place: r line (j,k) = (i, j) of the thread, s line (i,k)
+    // derivatives in place: r line (j,k) = (i, j) of the thread, s line (i,k); node n of either has
+    // the exponent of column (i,j) = (n, i) or (i, n)
     if (act) {
-      long long r[CQ];
-      int x[CQ];
-      long long* line = Ai + f * AS + j * PS + i * LQ;
+      auto derive = [&](long long* line, int stride, int from, int step, int* ex) {
+        Ln<CQ> l;
+        if (same) {
+          double v[CQ];
 #pragma unroll
-      for (int n = 0; n < CQ; ++n) {
-        r[n] = line[n];
-        x[n] = e3[f * CQ2 + i * CQ + n] + xI[j];
-      }
-      Ln<CQ> l;
-      l.from(r, x);
-      ok = l.fits(tD, CQ, S::RQ) && ok;
-      e1[tid] = l.x + l.kOut;
-#pragma unroll 2
-      for (int p = 0; p < CQ; ++p) line[p] = l.dot(tD + p * S::RQ);
-      line = Bi + f * AS + j * PS + i;
+          for (int n = 0; n < CQ; ++n) v[n] = __longlong_as_double(line[n * stride]);
+          ok = l.from(v, kULo, kUHi) && ok;
+        } else {
+          long long r[CQ];
+          int x[CQ];
 #pragma unroll
-      for (int n = 0; n < CQ; ++n) {
-        r[n] = line[n * LQ];
-        x[n] = e3[f * CQ2 + n * CQ + i] + xI[j];
-      }
-      l.from(r, x);
-      ok = l.fits(tD, CQ, S::RQ) && ok;
-      e2[tid] = l.x + l.kOut;
+          for (int n = 0; n < CQ; ++n) {
+            r[n] = line[n * stride];
+            x[n] = e3[from + n * step] + xI[j];
+          }
+          l.from(r, x);
+        }
+        ok = l.fits(tD, CQ, S::RQ) && ok;
+        ex[tid] = l.x + l.kOut;
 #pragma unroll 2
-      for (int p = 0; p < CQ; ++p) line[p * LQ] = l.dot(tD + p * S::RQ);
+        for (int p = 0; p < CQ; ++p) line[p * stride] = l.dot(tD + p * S::RQ);
+      };
+      derive(Ai + f * AS + j * PS + i * LQ, 1, f * CQ2 + i * CQ, 1, e1);
+      derive(Bi + f * AS + j * PS + i, LQ, f * CQ2 + i, CQ, e2);
     }
     __syncthreads();
     // advection term of the column, then its projection in t: A[f][c][j][i], exponent e3[(f,j,i)] + xIt[c]
@@ -390,17 +440,25 @@ k_adv_fx(int64_t E, const double* __restrict__ vgeo, const double* __restrict__ 
         const double dt = fx::to_double(t.dot(tD + k * S::RQ), xt + xD[k]);
         A[f * AS + n] = fma(H[2 * AS + n], dt, fma(H[AS + n], ds, H[n] * dr));
       }
-      double v[CQ];
+      if (!same) {
+        double v[CQ];
 #pragma unroll
-      for (int k = 0; k < CQ; ++k) v[k] = A[col + k * PS];
-      Ln<CQ> l;
-      ok = l.from(v, fx::kExpLo, fx::kExpHi) && l.fits(tIt, NQ, S::RQ) && ok;
-      e3[tid] = l.x + l.kOut;
+        for (int k = 0; k < CQ; ++k) v[k] = A[col + k * PS];
+        Ln<CQ> l;
+        ok = l.from(v, fx::kExpLo, fx::kExpHi, full) && l.fits(tIt, NQ, S::RQ) && ok;
+        e3[tid] = l.x + l.kOut;
 #pragma unroll 2
-      for (int c = 0; c < NQ; ++c) Ai[col + c * PS] = l.dot(tIt + c * S::RQ);
+        for (int c = 0; c < NQ; ++c) Ai[col + c * PS] = l.dot(tIt + c * S::RQ);
+      }
     }
     if (__syncthreads_or(!ok)) {
       direct<NQ, CQ>(vg, cg, cubD, cubInterpT, offset, Ue, NUe, A, B, H);
+      continue;
+    }
+    if (same) {
+      if (act)
+        for (int k = 0; k < CQ; ++k)
+          NUe[f * offset + k * CQ2 + ij] = vg[kIJW * Np + k * CQ2 + ij] * A[col + k * PS];
       continue;
     }
     // in s: line (f,c,i) in place, exponent e1[(f,c,i)] + xIt[b]
@@ -415,7 +473,7 @@ k_adv_fx(int64_t E, const double* __restrict__ vgeo, const double* __restrict__ 
         x[jj] = e3[ff * CQ2 + jj * CQ + ii] + xIt[c];
       }
       Ln<CQ> l;
-      l.from(r, x);
+      l.template from<true>(r, x, full);
       ok = l.fits(tIt, NQ, S::RQ) && ok;
       e1[tid] = l.x + l.kOut;
 #pragma unroll 2
@@ -434,7 +492,7 @@ k_adv_fx(int64_t E, const double* __restrict__ vgeo, const double* __restrict__ 
         x[ii] = e1[(ff * NQ + c) * CQ + ii] + xIt[b];
       }
       Ln<CQ> l;
-      l.from(r, x);
+      l.template from<true>(r, x, full);
       ok = l.fits(tIt, NQ, S::RQ) && ok;
 #pragma unroll 2
       for (int a = 0; a < NQ; ++a)
