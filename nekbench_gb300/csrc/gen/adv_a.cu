@@ -2,32 +2,24 @@
 #include "adv_fx.cuh"
 
 namespace nekb {
-namespace adv {
-// NEKB_FP64 and NEKB_FP64_SPLIT alike: the fixed-point operator keeps FP64's digits and is
-// faster than the double-float one at every size measured (1.02 to 2.7 times)
-template <int NQ, int CQ>
-int launch(bool, int64_t E, const double* vgeo, const double* cubvgeo, const double* cubD,
-           const double* cubInterpT, int64_t offset, const double* U, double* NU, cudaStream_t s)
-{
-  return adv_fx::launch<NQ, CQ>(E, vgeo, cubvgeo, cubD, cubInterpT, offset, U, NU, s);
-}
-template int launch<2, 2>(bool, int64_t, const double*, const double*, const double*, const double*, int64_t,
-                            const double*, double*, cudaStream_t);
-template int launch<3, 3>(bool, int64_t, const double*, const double*, const double*, const double*, int64_t,
-                            const double*, double*, cudaStream_t);
-template int launch<4, 4>(bool, int64_t, const double*, const double*, const double*, const double*, int64_t,
-                            const double*, double*, cudaStream_t);
-template int launch<5, 5>(bool, int64_t, const double*, const double*, const double*, const double*, int64_t,
-                            const double*, double*, cudaStream_t);
-template int launch<6, 6>(bool, int64_t, const double*, const double*, const double*, const double*, int64_t,
-                            const double*, double*, cudaStream_t);
-template int launch<7, 7>(bool, int64_t, const double*, const double*, const double*, const double*, int64_t,
-                            const double*, double*, cudaStream_t);
-template int launch<2, 3>(bool, int64_t, const double*, const double*, const double*, const double*, int64_t,
-                            const double*, double*, cudaStream_t);
-template int launch<3, 5>(bool, int64_t, const double*, const double*, const double*, const double*, int64_t,
-                            const double*, double*, cudaStream_t);
-template int launch<4, 6>(bool, int64_t, const double*, const double*, const double*, const double*, int64_t,
-                            const double*, double*, cudaStream_t);
-}  // namespace adv
+namespace adv_fx {
+template int launch<2, 2>(int64_t, const double*, const double*, const double*, const double*, int64_t,
+                           const double*, double*, cudaStream_t);
+template int launch<3, 3>(int64_t, const double*, const double*, const double*, const double*, int64_t,
+                           const double*, double*, cudaStream_t);
+template int launch<4, 4>(int64_t, const double*, const double*, const double*, const double*, int64_t,
+                           const double*, double*, cudaStream_t);
+template int launch<5, 5>(int64_t, const double*, const double*, const double*, const double*, int64_t,
+                           const double*, double*, cudaStream_t);
+template int launch<6, 6>(int64_t, const double*, const double*, const double*, const double*, int64_t,
+                           const double*, double*, cudaStream_t);
+template int launch<7, 7>(int64_t, const double*, const double*, const double*, const double*, int64_t,
+                           const double*, double*, cudaStream_t);
+template int launch<2, 3>(int64_t, const double*, const double*, const double*, const double*, int64_t,
+                           const double*, double*, cudaStream_t);
+template int launch<3, 5>(int64_t, const double*, const double*, const double*, const double*, int64_t,
+                           const double*, double*, cudaStream_t);
+template int launch<4, 6>(int64_t, const double*, const double*, const double*, const double*, int64_t,
+                           const double*, double*, cudaStream_t);
+}  // namespace adv_fx
 }  // namespace nekb

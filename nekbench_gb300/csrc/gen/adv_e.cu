@@ -4,14 +4,11 @@
 namespace nekb {
 namespace adv {
 // split = false: native FP64; true: double-float on the FP32 pipes
-template <int NQ, int CQ>
-int launch(bool split, int64_t E, const double* vgeo, const double* cubvgeo, const double* cubD,
-           const double* cubInterpT, int64_t offset, const double* U, double* NU, cudaStream_t s)
+int launch_10_15(bool split, int64_t E, const double* vgeo, const double* cubvgeo, const double* cubD,
+                 const double* cubInterpT, int64_t offset, const double* U, double* NU, cudaStream_t s)
 {
-  return split ? launch_p<NQ, CQ, DF>(E, vgeo, cubvgeo, cubD, cubInterpT, offset, U, NU, s)
-               : launch_p<NQ, CQ, F64>(E, vgeo, cubvgeo, cubD, cubInterpT, offset, U, NU, s);
+  return split ? launch_p<10, 15, DF>(E, vgeo, cubvgeo, cubD, cubInterpT, offset, U, NU, s)
+               : launch_p<10, 15, F64>(E, vgeo, cubvgeo, cubD, cubInterpT, offset, U, NU, s);
 }
-template int launch<10, 15>(bool, int64_t, const double*, const double*, const double*, const double*, int64_t,
-                            const double*, double*, cudaStream_t);
 }  // namespace adv
 }  // namespace nekb
