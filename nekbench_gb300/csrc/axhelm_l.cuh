@@ -127,8 +127,6 @@ struct CfgL {
   static constexpr bool TRI = (PREC == NEKB_FP32_TRILINEAR);
   static constexpr int SMEM = 2 * TAB * 4 + NSET * 2 * AS * 8 * NF + (TRI ? NSET * 24 * 8 + 2 * NQ * 4 : 0);
   // registers per thread the launch bounds aim at, by measurement (16.8 M nodes, lambda, us:
-  // N=7, one field, 80 / 96: 123.1 / 118.7; three fields, 112 / 168: 330 / 219)
-    // registers per thread the launch bounds aim at, by measurement (16.8 M nodes, lambda, us:
   // N=7, one field, 80 / 96 / 168: 130 / 125 / 143; three fields 386 / 317 / 240)
   static constexpr int REGS = NF == 1 ? (NQ <= 5 ? 64 : 96) : (NQ <= 7 ? 112 : 168);
   static constexpr int MINB = 65536 / (REGS * THREADS) > 0 ? 65536 / (REGS * THREADS) : 1;

@@ -811,7 +811,8 @@ int run_train(nekb_net* net, int64_t E, const float* in, const float* target, cu
   constexpr int SM = train_smem<NQ, C>();
   static SmemOptIn smem_opt;
   NEKB_TRY(smem_opt.ensure(k_net_train<NQ, C>, SM));
-  // persistent CTAs: as many as an SM's shared memory and 64 K registers hold
+  // CTAs that go on from element to element: as many as an SM's shared memory holds (and their
+  // partial sums have room for)
   constexpr int kFit = (227 * 1024) / (SM + 1024);
   constexpr int kPerSm = kFit < 1 ? 1 : kFit < kTrainPerSm ? kFit : kTrainPerSm;
   int64_t grid = (int64_t)(net->gblocks / kTrainPerSm) * kPerSm;
