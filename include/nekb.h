@@ -42,7 +42,11 @@ extern "C" {
 #define NEKB_AX_PARTIAL  4
 
 /* precision of an axhelm application */
-#define NEKB_FP64            0  /* ggeo/lambda/q/Aq double                                   */
+#define NEKB_FP64            0  /* ggeo/lambda/q/Aq double; contractions in block fixed point:
+                                   each is within (Nq + 2) 2^-54 of max|D| max|v| of its line,
+                                   and up to Nq = 5, or for a D without the symmetry of GLL
+                                   nodes, FP64 sums where a line's terms are far below that.
+                                   An element's result does not depend on the other elements */
 #define NEKB_FP32            1  /* ggeo/lambda/q/Aq float                                    */
 #define NEKB_BF16            2  /* ggeo and lambda bf16 storage, q/Aq float, FP32 arithmetic */
 #define NEKB_FP32_TRILINEAR  3  /* geometry from 24 trilinear coefficients per element

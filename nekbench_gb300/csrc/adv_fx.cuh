@@ -18,9 +18,9 @@
 // overlaid on them.
 //
 // E = 8192, us: N=7, cubN=11 FP64 FMAs 6060, double-float 3800, this 2966 (the integer multiply-add
-// pipe 35 % busy, FP64 17 %; one CTA per SM, whose passes alternate between the two); Gauss
-// nodes, N=7, cubN=7 792; the element's own nodes 1670, 1050, 334; N=2, cubN=2, 155,344 elements, own
-// nodes 2700, 1600, 310.  Requesting the next element's metric terms into L2 and unrolling the
+// pipe active 50 % of the time at 34 % of its instruction rate, FP64 17 %; one CTA per SM, whose
+// passes alternate between the two); Gauss nodes, N=7, cubN=7 792; the element's own nodes 1670,
+// 1050, 334; N=2, cubN=2, 155,344 elements, own nodes 2700, 1600, 291.  Requesting the next element's metric terms into L2 and unrolling the
 // pointwise passes changed nothing.
 //
 // An element with values that have no fixed-point form, and all elements when a matrix
