@@ -51,11 +51,11 @@
 // where one value is 2^lone(N) above all others), and a matrix with an entry beside its
 // diagonal (N = 2: any entry, and no line is looked at) that is more than 2^kDense below its
 // row's or column's largest.  (GLL nodes, N=2..4,
-// one node's lambda 1e12 times the others: 5.6e-7 of the terms without the rule, 3e-16 with
-// it.)  The even-odd form has no such rule: it adds v_m and v_m' before the products, as
-// the even-odd sums in FP64 that it stands for did, and they lose 2^-53 of the line's
-// largest value there (steep lines, exp(-20 x): 1e-15 to 3.8e-15 of the terms at N=5..13, this
-// form 1.5e-16 to 1.2e-15).
+// one node's lambda 1e12 times the others: 6e-7 to 6e-6 of the terms without the rule, 3.4e-16 to
+// 3.8e-16 with it.)  The even-odd form has no such rule: it adds v_m and v_m' before the
+// products, as the even-odd sums in FP64 that it stands for did, and they lose 2^-53 of the
+// line's largest value there (steep lines, exp(-20 x), N=5..13: 1.3e-15 to 2.9e-15 of the terms, this form
+// 2.8e-16 to 1.5e-15).
 #pragma once
 
 #include <cuda_runtime.h>
