@@ -36,10 +36,12 @@ namespace nekb {
 namespace {
 
 constexpr int RT = 256;           // threads per reduction block
-// 152 SMs x 4 with vector access: the FP64 sums of a block cost more than its waits.  A thread
-// keeps a running sum per component of the vector, so its chains are no longer than those of
-// twice as many blocks with scalar access, which is what that takes.
-constexpr int kMaxRedBlocks = 608, kMaxRedBlocksScalar = 1216;
+// 152 SMs x 4: the FP64 sums of a block cost more than its waits.  With vector access a thread
+// keeps a running sum per component, so its chains are no longer than those of twice as many
+// blocks with scalar access.  With scalar access the blocks grow to that number as soon as a
+// chain would have more than kChain terms (N=8, 378 elements, 2 terms: 25 us per mixed iteration,
+// 27.7 with 1077 blocks).
+constexpr int kMaxRedBlocks = 608, kMaxRedBlocksScalar = 1216, kChain = 8;
 // k_fcg_dots has ten sums per block: two blocks per SM, each thread with up to eleven loads in
 // flight (N=7, 13,824 elements, us per iteration of the learned solve: 606, with 608 blocks of 64
 // registers 622, of 99 registers 620); the chains are those of 1216 blocks with scalar access
@@ -624,7 +626,8 @@ __global__ void k_mask_set(int64_t Nm, const int32_t* ids, double v, double* q)
 // blocks of a reduction over n entries, V to an access
 inline unsigned red_grid(int64_t n, int V)
 {
-  const int64_t most = V > 1 ? kMaxRedBlocks : kMaxRedBlocksScalar;
+  int64_t most = kMaxRedBlocks;
+  if (V == 1) most = std::clamp<int64_t>((n + RT * kChain - 1) / (RT * kChain), kMaxRedBlocks, kMaxRedBlocksScalar);
   int64_t b = (n / V + RT - 1) / RT;
   if (b < 1) b = 1;
   if (b > most) b = most;
